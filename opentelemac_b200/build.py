@@ -6,6 +6,7 @@ The library is plain CUDA C++ with an extern "C" interface
 import os
 import subprocess
 import sys
+import tempfile
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -13,8 +14,9 @@ CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIBDIR, "libbief_b200.so")
 
-SOURCES = ["bief_api.cu", "bief_noalloc.cu"]
-HEADERS = ["bief_device.cuh", "bief_kernels.cuh", "bief_batch.cuh"]
+SOURCES = ["bief_api.cu", "bief_krylov.cu", "bief_noalloc.cu", "bief_resident.cu"]
+HEADERS = ["bief_device.cuh", "bief_kernels.cuh", "bief_batch.cuh", "bief_krylov.h",
+           "bief_resident.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -38,13 +40,21 @@ def build(force=False, verbose=False, defines=(), out=None):
     target = out or LIB
     if not force and not _stale(target, deps):
         return target
-    cmd = [nvcc(), *ARCH, "-O3", "-lineinfo", "-std=c++17", "-shared", "-Xcompiler", "-fPIC",
-           "-I", os.path.join(ROOT, "include"), *[f"-D{d}" for d in defines], "-o", target,
-           *srcs]
+    # the sources compile side by side, then link
+    base = [nvcc(), *ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC"]
+    opts = ["-I", os.path.join(ROOT, "include"), *[f"-D{d}" for d in defines]]
     if verbose:
-        cmd.insert(1, "-Xptxas=-v")
-        print(" ".join(cmd))
-    subprocess.run(cmd, check=True)
+        opts.insert(0, "-Xptxas=-v")
+    with tempfile.TemporaryDirectory(dir=LIBDIR) as tmp:
+        objs = [os.path.join(tmp, os.path.basename(f) + ".o") for f in srcs]
+        cmds = [[*base, *opts, "-c", f, "-o", o] for f, o in zip(srcs, objs)]
+        if verbose:
+            print("\n".join(" ".join(c) for c in cmds))
+        procs = [subprocess.Popen(c) for c in cmds]
+        for c, p in zip(cmds, [p.wait() for p in procs]):
+            if p:
+                raise subprocess.CalledProcessError(p, c)
+        subprocess.run([*base, "-shared", "-o", target, *objs], check=True)
     return target
 
 

@@ -16,6 +16,8 @@
 
 #include "../../include/bief_b200.h"
 #include "bief_batch.cuh"
+#include "bief_krylov.h"
+#include "bief_resident.h"
 
 using namespace bief;
 
@@ -86,6 +88,17 @@ struct bief_handle {
   double *d_brel = nullptr;
   double *d_bpart = nullptr;
   long long bpart_cap = 0;
+  // plan of the solvers that keep their search direction in shared memory
+  // (bief_resident.h): 0 not made yet, 1 made, -1 the mesh does not fit
+  int res_state = 0;
+  bool res_cl = false;
+  ResPart res = {};
+  int res_halo_max = 0, max_deg = 0, max_sgdeg = 0, smem_max = 0;
+  int *d_res_off = nullptr, *d_res_halo = nullptr;
+  unsigned *d_res_loc = nullptr;
+  unsigned short *d_seg_li = nullptr, *d_sg_li = nullptr, *d_sg_li2 = nullptr;
+  int res_shift = 0;  // binary32 local indices: 0 byte offsets, 2 element numbers
+  ushort2 *d_rec_li = nullptr;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   float solve_ms = 0.f, matvec_ms = 0.f;
   int mv_pending = 0;
@@ -192,42 +205,7 @@ void dispatch_mv(bief_handle *h, int td, bool sym, bool tr, const double *xm, co
 #undef MV_CASE
 }
 
-// Kernel of a method for TYPDIA code td, storage sto, dot-product mode
-// (comp: MODASS = 3, compensated) and residency (wide: twice the blocks per
-// SM, MINB = 2 CG_MIN_BLOCKS)
-#define KSEL1(k, STO_, C_, M_)                                                \
-  (td == DIA_Q ? (void *)k<DIA_Q, STO_, C_, M_>                                \
-               : td == DIA_I ? (void *)k<DIA_I, STO_, C_, M_> : (void *)k<DIA_0, STO_, C_, M_>)
-#define KSELM(k, M_)                                                          \
-  (sto == 3 ? (comp ? KSEL1(k, 3, true, M_) : KSEL1(k, 3, false, M_))         \
-            : (comp ? KSEL1(k, 1, true, M_) : KSEL1(k, 1, false, M_)))
-#define KSEL(k) (wide ? KSELM(k, 2 * CG_MIN_BLOCKS) : KSELM(k, CG_MIN_BLOCKS))
-
 void *cg_kernel(int td, int sto, bool comp = false, bool wide = false) { return KSEL(k_cg64); }
-
-void *equnor_kernel(int td, int sto, bool comp = false, bool wide = false) {
-  return KSEL(k_equnor);
-}
-
-void *rescjg_kernel(int td, int sto, bool comp = false, bool wide = false) {
-  return KSEL(k_rescjg);
-}
-
-void *errmin_kernel(int td, int sto, bool comp = false, bool wide = false) {
-  return KSEL(k_errmin);
-}
-
-void *cgsqua_kernel(int td, int sto, bool comp = false, bool wide = false) {
-  return KSEL(k_cgsqua);
-}
-
-void *gmres_kernel(int td, int sto, bool comp = false, bool wide = false) {
-  return KSEL(k_gmres);
-}
-
-void *cgstab_kernel(int td, int sto, bool comp = false, bool wide = false) {
-  return KSEL(k_cgstab);
-}
 
 // ... and, for the binary32 kernels, c16: the slots' neighbours as 16-bit
 // offsets
@@ -402,9 +380,163 @@ int build_seg_coefs(bief_handle *h, const double *xa, cudaStream_t st) {
   return BIEF_OK;
 }
 
+static int res_mixed_vecs(const bief_handle *h);
+// ---------------------------------------------------------------------------
+// Plan of the resident solvers: who owns which node and what each block's
+// halo is, made at the first solve that can use it (and again when the
+// dot-product tree's shape or the segment numbering changes).
+// ---------------------------------------------------------------------------
+void res_drop(bief_handle *h) {
+  void *bufs[] = {h->d_res_off, h->d_res_halo, h->d_res_loc, h->d_seg_li, h->d_sg_li, h->d_sg_li2,
+                  h->d_rec_li};
+  for (void *p : bufs)
+    if (p) cudaFree(p);
+  h->d_res_off = h->d_res_halo = nullptr;
+  h->d_res_loc = nullptr;
+  h->d_seg_li = h->d_sg_li = h->d_sg_li2 = nullptr;
+  h->d_rec_li = nullptr;
+  h->res_state = 0;
+}
+
+int res_ensure(bief_handle *h, cudaStream_t st) {
+  if (h->res_state) return BIEF_OK;
+  h->res_state = -1;
+  if (h->max_deg > 255 || h->max_nnb > 255 || (h->has_segments && h->max_sgdeg > 255))
+    return BIEF_OK;
+  ResPart Q = {};
+  Q.n = h->npoin;
+  Q.G = h->G;
+  Q.S = Q.V = 1;
+  Q.R = 0;
+  for (int b = 0; b < Q.G; ++b) {
+    const long long lo = b ? ((long long)b * Q.n / Q.G) & ~31LL : 0;
+    const long long hi = b + 1 >= Q.G ? Q.n : (((long long)(b + 1) * Q.n / Q.G) & ~31LL);
+    Q.R = std::max(Q.R, (int)((hi - lo + RES_T - 1) / RES_T));
+  }
+  // Up to 16 tree blocks (32,768 nodes): one cluster, each tree block's warps
+  // shared out over as many of its blocks as there are.
+  h->res_cl = false;
+  if (Q.G <= RES_MAXCL && Q.R <= 2) {
+    int S = 1;
+    while (Q.G * 2 * S <= RES_MAXCL) S *= 2;
+    if (res_cluster_fits(Q.G * S, RES_T / S, (size_t)h->smem_max)) {
+      Q.S = S;
+      h->res_cl = true;
+    }
+  }
+  Q.TP = RES_T / Q.S;
+  if (Q.G > h->nsm) Q.V = (Q.G + h->nsm - 1) / h->nsm;
+  if (Q.V > 2) return BIEF_OK;
+  Q.NP = Q.V > 1 ? (Q.G + Q.V - 1) / Q.V : Q.G * Q.S;
+  Q.own = Q.V * Q.R * Q.TP;
+  if (Q.own > 0xffff) return BIEF_OK;
+  int stt;
+  if ((stt = dalloc(&h->d_res_off, (size_t)Q.NP + 1))) return stt;
+  Q.halo_off = h->d_res_off;
+  PlanP A = {};
+  A.Q = Q;
+  A.meta = h->d_meta;
+  A.seg_off = h->d_seg_off;
+  A.seg_col = h->d_seg_col;
+  A.rec_off = h->d_rec_off;
+  A.rec_idx = h->d_rec_idx;
+  A.halo_n = h->d_res_off;
+  CK(res_launch_plan(false, A, st));
+  std::vector<int> cnt(Q.NP + 1, 0);
+  CK(cudaMemcpyAsync(cnt.data(), h->d_res_off, sizeof(int) * Q.NP, cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  int total = 0, most = 0;
+  for (int p = 0; p <= Q.NP; ++p) {
+    const int c = p < Q.NP ? cnt[p] : 0;
+    most = std::max(most, c);
+    cnt[p] = total;
+    total += c;
+  }
+  if (Q.own + most > 0xffff) return BIEF_OK;
+  const bool sg = h->has_segments != 0;
+  if ((stt = dalloc(&h->d_res_halo, (size_t)total)) || (stt = dalloc(&h->d_res_loc, (size_t)total)) ||
+      (stt = dalloc(&h->d_seg_li, (size_t)h->nseg)) || (stt = dalloc(&h->d_rec_li, (size_t)h->nrec + 32)) ||
+      (sg && ((stt = dalloc(&h->d_sg_li, (size_t)h->nsg_slots + 32)) ||
+              (stt = dalloc(&h->d_sg_li2, (size_t)h->nsg_slots)))))
+    return stt;
+  CK(cudaMemcpyAsync(h->d_res_off, cnt.data(), sizeof(int) * (Q.NP + 1), cudaMemcpyHostToDevice,
+                     st));
+  CK(cudaMemsetAsync(h->d_seg_li, 0, sizeof(short) * h->nseg, st));
+  CK(cudaMemsetAsync(h->d_rec_li, 0, sizeof(ushort2) * (h->nrec + 32), st));
+  if (sg) {
+    CK(cudaMemsetAsync(h->d_sg_li, 0, sizeof(short) * (h->nsg_slots + 32), st));
+    CK(cudaMemsetAsync(h->d_sg_li2, 0, sizeof(short) * h->nsg_slots, st));
+  }
+  // binary32 windows: local indices as byte offsets while those fit 16 bits
+  // (and the vectors stand in shared memory: the kernel forms that exist)
+  h->res = Q;
+  h->res_halo_max = most;
+  h->res_shift = 4LL * (Q.own + most) <= 0xffff && res_mixed_vecs(h) ? 0 : 2;
+  A.shift = 2 - h->res_shift;
+  A.halo = h->d_res_halo;
+  A.halo_loc = h->d_res_loc;
+  A.seg_li = h->d_seg_li;
+  A.rec_li = h->d_rec_li;
+  if (sg) {
+    A.sg_li = h->d_sg_li;
+    A.sg_li2 = h->d_sg_li2;
+    A.sg_meta = h->d_sg_meta;
+    A.sg_off = h->d_sg_off;
+    A.sg_col = h->d_sg_col;
+  }
+  CK(res_launch_plan(true, A, st));
+  CK(cudaStreamSynchronize(st));
+  h->launches += 2;
+  Q.halo = h->d_res_halo;
+  Q.halo_loc = h->d_res_loc;
+  h->res = Q;
+  h->res_halo_max = most;
+  h->res_state = 1;
+  return BIEF_OK;
+}
+
+// Slots of the operator kept in shared memory beside a layout of `base`
+// bytes: as many whole 32-slot rows as the rest holds.
+static int res_cache_slots(const bief_handle *h, size_t base, int bytes_per_slot) {
+  const long long room = (long long)h->smem_max - (long long)base - 64;
+  if (room <= 0) return 0;
+  const long long most = 16LL * h->res.own;
+  return (int)(std::min(room / bytes_per_slot, most) / 32 * 32);
+}
+
 // Transposed-operator coefficients for EQUNOR ('Q' storage; symmetric
 // storage reuses the operator's own).  Returns the Sell of A^T.
 int build_transposed(bief_handle *h, const double *xm, cudaStream_t st, Sell *out);
+
+// Binary32 copy of the working operator (xm, da) for the mixed solvers: slot
+// coefficients and row sums; pair: the slots in pairs (bief_resident.cu).
+// Segment storage takes them from the binary64 slots (build_seg_coefs).
+int build_slots32(bief_handle *h, int td, const double *xm, const double *da, bool pair,
+                  cudaStream_t s) {
+  const int gn = grid_for(h->npoin, h->nsm);
+#define SLOTS32(k, ...)                                                              \
+  do {                                                                               \
+    if (td == DIA_Q)                                                                 \
+      pair ? k<DIA_Q, true><<<gn, 256, 0, s>>>(__VA_ARGS__)                          \
+           : k<DIA_Q, false><<<gn, 256, 0, s>>>(__VA_ARGS__);                        \
+    else if (td == DIA_I)                                                            \
+      pair ? k<DIA_I, true><<<gn, 256, 0, s>>>(__VA_ARGS__)                          \
+           : k<DIA_I, false><<<gn, 256, 0, s>>>(__VA_ARGS__);                        \
+    else                                                                             \
+      pair ? k<DIA_0, true><<<gn, 256, 0, s>>>(__VA_ARGS__)                          \
+           : k<DIA_0, false><<<gn, 256, 0, s>>>(__VA_ARGS__);                        \
+  } while (0)
+  if (h->sto == 3)
+    SLOTS32(k_build_sg32, h->npoin, h->d_sg_meta, h->d_sg_off, h->d_sg_c64, da, h->d_sg_c32,
+            h->d_s32);
+  else
+    SLOTS32(k_build_seg32, h->npoin, h->nelem, h->d_ptr, h->d_ek, xm, da, h->d_meta,
+            h->d_rec_off, h->d_rec_slot, h->d_seg_off, h->d_seg_c, h->d_s32);
+#undef SLOTS32
+  h->launches++;
+  CK(cudaGetLastError());
+  return BIEF_OK;
+}
 
 // Operator loads are marked evict-first when the kernel's working set --
 // the operator stream plus the node vectors the solvers keep (binary64:
@@ -477,6 +609,104 @@ int build_transposed(bief_handle *h, const double *xm, cudaStream_t st, Sell *ou
   h->launches++;
   CK(cudaGetLastError());
   *out = S;
+  return BIEF_OK;
+}
+
+// GRACJG with the search direction in shared memory; *done = false when the
+// mesh's window does not fit (k_cg64 then).
+int res_cg(bief_handle *h, const CgP &C, int td, cudaStream_t s, bool *done) {
+  *done = false;
+  int st = res_ensure(h, s);
+  if (st || h->res_state != 1) return st;
+  const ResPart &Q = h->res;
+  const int cb = h->sto == 3 ? 8 : 16, ib = h->sto == 3 ? 2 : 4;
+  int nvec = h->res_cl ? 3 : 2;  // R, AD (and X) of the own rows
+  size_t base = res_layout(Q.own, h->res_halo_max, Q.G, h->res_cl, 8, nvec, cb, ib, 0).total;
+  if (base > (size_t)h->smem_max) {
+    if (h->res_cl) return BIEF_OK;
+    nvec = 0;
+    base = res_layout(Q.own, h->res_halo_max, Q.G, h->res_cl, 8, nvec, cb, ib, 0).total;
+    if (base > (size_t)h->smem_max) return BIEF_OK;
+  }
+  ResP P = {};
+  P.Q = Q;
+  P.S = C.S;
+  P.li = h->d_sg_li;
+  P.rli = h->d_rec_li;
+  P.td = td;
+  P.da = C.da;
+  P.dsc = C.dsc;
+  P.x = C.x;
+  P.b = C.b;
+  P.ctl = C.ctl;
+  P.part = C.part;
+  P.timeout_ns = C.timeout_ns;
+  P.cache = res_cache_slots(h, base, cb + ib);
+  P.halo_max = h->res_halo_max;
+  P.nitmax = C.nitmax;
+  P.nvec = nvec;
+  P.eps = C.eps;
+  // An operator larger than the L2: the slots of the leading steps, 0.45 of
+  // the L2 in all, are loaded to stay there, the others stream through it
+  // (1.0M nodes, 7 steps of 17 MB: 30.1 us per iteration with every step
+  // streamed, 28.2 / 27.4 / 27.2 / 28.9 / 33.0 with 1 to 5 steps kept).
+  const double op = (cb + ib) * (double)(h->sto == 3 ? h->nsg_slots : h->nrec);
+  P.keep = C.S.cs_rec ? (int)(0.45 * h->l2_bytes / (op / (Q.V * Q.R))) : Q.V * Q.R;
+  P.r = C.r;
+  P.ad = C.ad;
+  const size_t smem =
+      res_layout(Q.own, h->res_halo_max, Q.G, h->res_cl, 8, nvec, cb, ib, P.cache).total;
+  CK(res_launch_cg(h->sto, h->res_cl, P, smem, s));
+  h->launches++;
+  *done = true;
+  return BIEF_OK;
+}
+
+// The mixed-precision solve likewise: r, q, z and the row sums of the own
+// rows in shared memory when they fit (always in the cluster form), else in
+// global memory.
+static size_t res_mixed_layout(const bief_handle *h, int nvec, int cache) {
+  return res_layout(h->res.own, h->res_halo_max, h->res.G, h->res_cl, 4, nvec, 4, 2, cache).total;
+}
+static int res_mixed_vecs(const bief_handle *h) {
+  return res_mixed_layout(h, 4, 0) <= (size_t)h->smem_max ? 4 : 0;
+}
+bool res_mixed_fits(const bief_handle *h) {
+  if (h->res_state != 1) return false;
+  const int nvec = res_mixed_vecs(h);
+  if (h->res_cl && (nvec == 0 || h->res_shift)) return false;
+  return res_mixed_layout(h, nvec, 0) <= (size_t)h->smem_max;
+}
+
+int res_mixed(bief_handle *h, const MixP &C, int td, cudaStream_t s) {
+  const ResPart &Q = h->res;
+  const int nvec = res_mixed_vecs(h);
+  const size_t base = res_mixed_layout(h, nvec, 0);
+  ResP P = {};
+  P.Q = Q;
+  P.S = C.S;
+  P.li = h->sto == 3 ? h->d_sg_li2 : h->d_seg_li;
+  P.td = td;
+  P.da = C.da;
+  P.dsc = C.dsc;
+  P.x = C.x;
+  P.b = C.b;
+  P.ctl = C.ctl;
+  P.part = C.part;
+  P.timeout_ns = C.timeout_ns;
+  P.cache = res_cache_slots(h, base, 6) / 64 * 64;
+  P.nvec = nvec;
+  P.halo_max = h->res_halo_max;
+  P.max_outer = C.max_outer;
+  P.max_inner = C.max_inner;
+  P.outer_tol = C.outer_tol;
+  P.inner_tol = C.inner_tol;
+  P.z = C.z;
+  P.ri = C.ri;
+  P.q = C.q;
+  CK(res_launch_mixed(h->sto, h->res_cl, nvec == 4, h->res_shift, P,
+                      res_mixed_layout(h, nvec, P.cache), s));
+  h->launches++;
   return BIEF_OK;
 }
 
@@ -580,6 +810,7 @@ int bief_mesh_create(int npoin, int nelem, int nelmax, const int *ikle, int devi
       wr = std::max(wr, ptr[i + 1] - ptr[i]);
       ws = std::max(ws, nnb[i]);
     }
+    ws = (ws + 1) & ~1;  // binary32 slots also stand in pairs (bief_resident.h)
     const long long r = (long long)rec_off[sgi] + 32LL * wr, q = (long long)seg_off[sgi] + 32LL * ws;
     if (r > 0x7fffffffLL || q > 0x7fffffffLL) return BIEF_ERR_SIZE;
     rec_off[sgi + 1] = (int)r;
@@ -672,6 +903,7 @@ int bief_mesh_create(int npoin, int nelem, int nelmax, const int *ikle, int devi
   h->nrec = (long long)nrec;
   h->nseg = (long long)nseg;
   h->max_nnb = max_nnb;
+  for (int i = 0; i < npoin; ++i) h->max_deg = std::max(h->max_deg, ptr[i + 1] - ptr[i]);
   int st = BIEF_OK;
   {
     DevGuard g(device);
@@ -681,6 +913,9 @@ int bief_mesh_create(int npoin, int nelem, int nelmax, const int *ikle, int devi
     if ((e = cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess)
       return fail(cuda_fail(e, "cudaDeviceGetAttribute", __LINE__));
     if ((e = cudaDeviceGetAttribute(&h->l2_bytes, cudaDevAttrL2CacheSize, device)) != cudaSuccess)
+      return fail(cuda_fail(e, "cudaDeviceGetAttribute", __LINE__));
+    if ((e = cudaDeviceGetAttribute(&h->smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin,
+                                    device)) != cudaSuccess)
       return fail(cuda_fail(e, "cudaDeviceGetAttribute", __LINE__));
     if ((e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking)) != cudaSuccess)
       return fail(cuda_fail(e, "cudaStreamCreate", __LINE__));
@@ -698,7 +933,7 @@ int bief_mesh_create(int npoin, int nelem, int nelmax, const int *ikle, int devi
         (st = dalloc(&h->d_ctl, 1)) || (st = dalloc(&h->d_meta, n)) ||
         (st = dalloc(&h->d_rec_off, (size_t)nsl + 1)) || (st = dalloc(&h->d_seg_off, (size_t)nsl + 1)) ||
         (st = dalloc(&h->d_rec_idx, nrec)) || (st = dalloc(&h->d_rec_slot, nrec)) ||
-        (st = dalloc(&h->d_rec_c, nrec)) || (st = dalloc(&h->d_seg_col, nseg)) ||
+        (st = dalloc(&h->d_rec_c, nrec + 32)) || (st = dalloc(&h->d_seg_col, nseg)) ||
         (st = dalloc(&h->d_seg_c, nseg)))
       return fail(st);
     if (mvf != MV_NONE) {
@@ -755,7 +990,7 @@ int bief_mesh_create(int npoin, int nelem, int nelmax, const int *ikle, int devi
         (e = cudaMemcpyAsync(h->d_seg_col, seg_col.data(), sizeof(int) * nseg,
                              cudaMemcpyHostToDevice, h->stream)) != cudaSuccess ||
         (e = cudaMemsetAsync(h->d_seg_c, 0, sizeof(float) * nseg, h->stream)) != cudaSuccess ||
-        (e = cudaMemsetAsync(h->d_rec_c, 0, sizeof(double2) * nrec, h->stream)) != cudaSuccess ||
+        (e = cudaMemsetAsync(h->d_rec_c, 0, sizeof(double2) * (nrec + 32), h->stream)) != cudaSuccess ||
         (e = cudaStreamSynchronize(h->stream)) != cudaSuccess)
       return fail(cuda_fail(e, "mesh upload", __LINE__));
   }
@@ -767,6 +1002,7 @@ int bief_destroy(bief_handle *h) {
   if (!h) return BIEF_ERR_ARGS;
   DevGuard g(h->dev);
   if (h->stream) cudaStreamSynchronize(h->stream);
+  res_drop(h);
   void *bufs[] = {h->d_ptr, h->d_ek, h->d_ik, h->d_dm, h->d_xm, h->d_dms, h->d_xms, h->d_dsc,
                   h->d_s32, h->d_x, h->d_b, h->d_bs, h->d_r, h->d_d0, h->d_d1,
                   h->d_ad, h->d_t, h->d_z, h->d_ri, h->d_p0, h->d_p1, h->d_q, h->d_part,
@@ -1036,8 +1272,11 @@ int bief_solve_dev(bief_handle *h, double *x, double *b, bief_slvcfg *cfg, int f
     P.part = h->d_part;
     P.ctl = h->d_ctl;
     P.timeout_ns = h->timeout_ns;
+    bool done = false;
+    if (!comp && (st = res_ensure(h, s))) return st;  // plan outside the timed launch
     CK(cudaEventRecord(h->ev[0], s));
-    if ((st = launch_coop(h, cg_kernel(td, h->sto, comp, h->wide), &P, s))) return st;
+    if (!comp && (st = res_cg(h, P, td, s, &done))) return st;
+    if (!done && (st = launch_coop(h, cg_kernel(td, h->sto, comp, h->wide), &P, s))) return st;
   }
   CK(cudaEventRecord(h->ev[1], s));
   CK(cudaMemcpyAsync(h->h_ctl, h->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
@@ -1116,39 +1355,11 @@ int bief_solve_mixed_dev(bief_handle *h, double *x, const double *b, int precon,
     da = h->d_dms;
     bw = h->d_bs;
   }
-  if (seg) {
-    // binary64 slot coefficients, then their binary32 copy and row sums
-    if ((st = build_seg_coefs(h, xm, s))) return st;
-    const int gn = grid_for(h->npoin, h->nsm);
-#define SG_ARGS h->npoin, h->d_sg_meta, h->d_sg_off, h->d_sg_c64, da, h->d_sg_c32, h->d_s32
-    if (td == DIA_Q)
-      k_build_sg32<DIA_Q><<<gn, 256, 0, s>>>(SG_ARGS);
-    else if (td == DIA_I)
-      k_build_sg32<DIA_I><<<gn, 256, 0, s>>>(SG_ARGS);
-    else
-      k_build_sg32<DIA_0><<<gn, 256, 0, s>>>(SG_ARGS);
-#undef SG_ARGS
-    h->launches++;
-    h->s32_gen = -1;
-    CK(cudaGetLastError());
-  } else if ((st = build_records(h, xm, s))) {
-    return st;
-  } else {  // binary32 edge-assembled copy of the working operator
-    const int gn = grid_for(h->npoin, h->nsm);
-#define SEG_ARGS                                                                              \
-  h->npoin, h->nelem, h->d_ptr, h->d_ek, xm, da, h->d_meta, h->d_rec_off, h->d_rec_slot, \
-      h->d_seg_off, h->d_seg_c, h->d_s32
-    if (td == DIA_Q)
-      k_build_seg32<DIA_Q><<<gn, 256, 0, s>>>(SEG_ARGS);
-    else if (td == DIA_I)
-      k_build_seg32<DIA_I><<<gn, 256, 0, s>>>(SEG_ARGS);
-    else
-      k_build_seg32<DIA_0><<<gn, 256, 0, s>>>(SEG_ARGS);
-#undef SEG_ARGS
-    h->launches++;
-    h->s32_gen = -1;
-    CK(cudaGetLastError());
-  }
+  if ((st = res_ensure(h, s))) return st;
+  const bool pair = res_mixed_fits(h);  // slots in pairs for k_mixed_res
+  if ((st = seg ? build_seg_coefs(h, xm, s) : build_records(h, xm, s))) return st;
+  if ((st = build_slots32(h, td, xm, da, pair, s))) return st;
+  h->s32_gen = -1;
   MixP P;
   P.npoin = h->npoin;
   P.max_outer = max_outer;
@@ -1170,7 +1381,9 @@ int bief_solve_mixed_dev(bief_handle *h, double *x, const double *b, int precon,
   P.timeout_ns = h->timeout_ns;
   CK(cudaMemsetAsync(h->d_ctl, 0, sizeof(Ctl), s));
   CK(cudaEventRecord(h->ev[0], s));
-  if ((st = launch_coop(h, mixed_kernel(td, h->sto, h->wide, slots16(h)), &P, s))) return st;
+  if ((st = pair ? res_mixed(h, P, td, s)
+                 : launch_coop(h, mixed_kernel(td, h->sto, h->wide, slots16(h)), &P, s)))
+    return st;
   CK(cudaEventRecord(h->ev[1], s));
   CK(cudaMemcpyAsync(h->h_ctl, h->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
@@ -1257,33 +1470,11 @@ int bief_matvec32_dev(bief_handle *h, float *x, const float *y, void *stream) {
   if (!seg && h->max_nnb > MAX_NEIGHBOURS) return BIEF_ERR_SIZE;
   DevGuard g(h->dev);
   cudaStream_t s = (cudaStream_t)stream;
-  const int td = typdia_code(h->typdia), gn = grid_for(h->npoin, h->nsm);
+  const int td = typdia_code(h->typdia);
   if (h->s32_gen != h->mat_gen) {  // binary32 copy of the stored matrix
     int st;
-    if (seg) {
-      if ((st = build_seg_coefs(h, h->d_xa, s))) return st;
-#define SG_ARGS h->npoin, h->d_sg_meta, h->d_sg_off, h->d_sg_c64, h->d_dm, h->d_sg_c32, h->d_s32
-      if (td == DIA_Q)
-        k_build_sg32<DIA_Q><<<gn, 256, 0, s>>>(SG_ARGS);
-      else if (td == DIA_I)
-        k_build_sg32<DIA_I><<<gn, 256, 0, s>>>(SG_ARGS);
-      else
-        k_build_sg32<DIA_0><<<gn, 256, 0, s>>>(SG_ARGS);
-#undef SG_ARGS
-    } else {
-#define SEG_ARGS                                                                               \
-  h->npoin, h->nelem, h->d_ptr, h->d_ek, h->d_xm, h->d_dm, h->d_meta, h->d_rec_off,           \
-      h->d_rec_slot, h->d_seg_off, h->d_seg_c, h->d_s32
-      if (td == DIA_Q)
-        k_build_seg32<DIA_Q><<<gn, 256, 0, s>>>(SEG_ARGS);
-      else if (td == DIA_I)
-        k_build_seg32<DIA_I><<<gn, 256, 0, s>>>(SEG_ARGS);
-      else
-        k_build_seg32<DIA_0><<<gn, 256, 0, s>>>(SEG_ARGS);
-#undef SEG_ARGS
-    }
-    h->launches++;
-    CK(cudaGetLastError());
+    if (seg && (st = build_seg_coefs(h, h->d_xa, s))) return st;
+    if ((st = build_slots32(h, td, h->d_xm, h->d_dm, false, s))) return st;
     h->s32_gen = h->mat_gen;
   }
   if (x == y) {  // as MATVEC, X may alias Y
@@ -1480,40 +1671,9 @@ int bief_batch_solve_mixed_dev(bief_handle *h, int ninst, const int *node_off,
     da = h->d_dms;
     bw = h->d_bs;
   }
-  if (seg) {
-    // segment storage: binary64 slot coefficients, their binary32 copy and
-    // row sums, as the single-mesh mixed solve builds them
-    if ((st = build_seg_coefs(h, xm, s))) return st;
-    const int gn = grid_for(h->npoin, h->nsm);
-#define SG_ARGS h->npoin, h->d_sg_meta, h->d_sg_off, h->d_sg_c64, da, h->d_sg_c32, h->d_s32
-    if (td == DIA_Q)
-      k_build_sg32<DIA_Q><<<gn, 256, 0, s>>>(SG_ARGS);
-    else if (td == DIA_I)
-      k_build_sg32<DIA_I><<<gn, 256, 0, s>>>(SG_ARGS);
-    else
-      k_build_sg32<DIA_0><<<gn, 256, 0, s>>>(SG_ARGS);
-#undef SG_ARGS
-    h->launches++;
-    h->s32_gen = -1;
-    CK(cudaGetLastError());
-  } else if ((st = build_records(h, xm, s))) {
-    return st;
-  } else {
-    const int gn = grid_for(h->npoin, h->nsm);
-#define SEG_ARGS                                                                              \
-  h->npoin, h->nelem, h->d_ptr, h->d_ek, xm, da, h->d_meta, h->d_rec_off, h->d_rec_slot, \
-      h->d_seg_off, h->d_seg_c, h->d_s32
-    if (td == DIA_Q)
-      k_build_seg32<DIA_Q><<<gn, 256, 0, s>>>(SEG_ARGS);
-    else if (td == DIA_I)
-      k_build_seg32<DIA_I><<<gn, 256, 0, s>>>(SEG_ARGS);
-    else
-      k_build_seg32<DIA_0><<<gn, 256, 0, s>>>(SEG_ARGS);
-#undef SEG_ARGS
-    h->launches++;
-    h->s32_gen = -1;
-    CK(cudaGetLastError());
-  }
+  if ((st = seg ? build_seg_coefs(h, xm, s) : build_records(h, xm, s))) return st;
+  if ((st = build_slots32(h, td, xm, da, false, s))) return st;
+  h->s32_gen = -1;
   void *k = batch_kernel(td, seg ? 3 : 1, h->wide, seg ? h->sg16 : h->seg16);
   int bps = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k, threads_per_block, 0));
@@ -1693,6 +1853,7 @@ int bief_set_blocks_per_sm(bief_handle *h, int blocks_per_sm) {
   if ((st = persistent_grid(h->npoin, h->nsm, wide, &G))) return st;
   if (G != h->G) {
     CK(cudaStreamSynchronize(h->stream));
+    res_drop(h);
     CK(cudaFree(h->d_part));
     h->d_part = nullptr;
     if (h->d_gpart) CK(cudaFree(h->d_gpart));  // sized by G at its first use
@@ -1764,6 +1925,7 @@ int bief_set_segments(bief_handle *h, int nseg, int maxseg, const int *gloseg) {
   for (int sl = 0; sl < nsl; ++sl) {
     int w = 0;
     for (int i = 32 * sl; i < std::min(n, 32 * sl + 32); ++i) w = std::max(w, deg[i]);
+    w = (w + 1) & ~1;  // as the element storage's binary32 slots
     const long long o = (long long)off[sl] + 32LL * w;
     if (o > 0x7fffffffLL) return BIEF_ERR_SIZE;
     off[sl + 1] = (int)o;
@@ -1791,6 +1953,7 @@ int bief_set_segments(bief_handle *h, int nseg, int maxseg, const int *gloseg) {
                  h->d_sg_dc, h->d_segel, h->d_xa, h->d_xas, h->d_sg_c64, h->d_sg_c32,
                  h->d_sg_ct};
   CK(cudaStreamSynchronize(h->stream));
+  res_drop(h);
   for (void *p : old)
     if (p) cudaFree(p);
   h->d_g1 = h->d_g2 = h->d_sg_meta = h->d_sg_off = h->d_sg_sx = h->d_sg_col = nullptr;
@@ -1808,7 +1971,7 @@ int bief_set_segments(bief_handle *h, int nseg, int maxseg, const int *gloseg) {
       (st = dalloc(&h->d_sg_meta, n)) || (st = dalloc(&h->d_sg_off, (size_t)nsl + 1)) ||
       (st = dalloc(&h->d_sg_sx, nslot)) || (st = dalloc(&h->d_sg_col, nslot)) ||
       (st = dalloc(&h->d_segel, nseg)) || (st = dalloc(&h->d_xa, 2 * (size_t)nseg)) ||
-      (st = dalloc(&h->d_xas, 2 * (size_t)nseg)) || (st = dalloc(&h->d_sg_c64, nslot)) ||
+      (st = dalloc(&h->d_xas, 2 * (size_t)nseg)) || (st = dalloc(&h->d_sg_c64, nslot + 32)) ||
       (st = dalloc(&h->d_sg_c32, nslot)))
     return st;
   CK(cudaMemcpyAsync(h->d_g1, g1.data(), sizeof(int) * nseg, cudaMemcpyHostToDevice, h->stream));
@@ -1823,7 +1986,7 @@ int bief_set_segments(bief_handle *h, int nseg, int maxseg, const int *gloseg) {
                      h->stream));
   CK(cudaMemcpyAsync(h->d_segel, segel.data(), sizeof(int2) * nseg, cudaMemcpyHostToDevice,
                      h->stream));
-  CK(cudaMemsetAsync(h->d_sg_c64, 0, sizeof(double) * nslot, h->stream));
+  CK(cudaMemsetAsync(h->d_sg_c64, 0, sizeof(double) * (nslot + 32), h->stream));
   CK(cudaMemsetAsync(h->d_sg_c32, 0, sizeof(float) * nslot, h->stream));
   if (fit16) {  // the binary32 kernels read 2-byte offsets instead of the columns
     if ((st = dalloc(&h->d_sg_dc, nslot))) return st;
@@ -1833,6 +1996,7 @@ int bief_set_segments(bief_handle *h, int nseg, int maxseg, const int *gloseg) {
   CK(cudaStreamSynchronize(h->stream));
   h->sg16 = fit16;
   h->nsg = nseg;
+  h->max_sgdeg = *std::max_element(deg.begin(), deg.end());
   h->nsg_slots = (long long)nslot;
   h->has_segments = 1;
   return BIEF_OK;

@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(256) k_mvseg(int npoin, int nseg, bool ext,
 
 // OMSEG 'M=DMD' off-diagonal part (omseg.f:530-541):
 // XA(ISEG) * D(GLOSEG1) * D(GLOSEG2), for each stored column.
-__global__ void k_precd1_segs(int nseg, int ncol, const int *__restrict__ g1,
+static __global__ void k_precd1_segs(int nseg, int ncol, const int *__restrict__ g1,
                               const int *__restrict__ g2, const double *__restrict__ dsc,
                               const double *__restrict__ xa, double *xas) {
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nseg; s += gridDim.x * blockDim.x) {
@@ -295,7 +295,16 @@ __global__ void k_build_sgc(int npoin, int nseg, const int *__restrict__ meta,
 // Binary32 operator of a symmetric segment matrix for the mixed solver: the
 // slot coefficients rounded, and the row sum diag + XA of each slot added
 // in slot order in binary64, rounded once.
-template <int TD>
+//
+// PAIR: the slots in pairs, as bief_resident.cu reads them (slot m of a lane
+// at float2 m / 2 of the slice).
+template <bool PAIR>
+__device__ __forceinline__ int slot_at(int i, int base, int m) {
+  if (!PAIR) return base + 32 * m;
+  return 2 * (((base - (i & 31)) >> 1) + 32 * (m >> 1) + (i & 31)) + (m & 1);
+}
+
+template <int TD, bool PAIR = false>
 __global__ void k_build_sg32(int npoin, const int *__restrict__ meta, const int *__restrict__ off,
                              const double *__restrict__ sg_c, const double *__restrict__ da,
                              float *seg_c, float *s32) {
@@ -305,7 +314,7 @@ __global__ void k_build_sg32(int npoin, const int *__restrict__ meta, const int 
     double srow = TD == DIA_Q ? da[i] : (TD == DIA_I ? 1.0 : 0.0);
     for (int m = 0; m < deg; ++m) {
       const double cv = sg_c[base + 32 * m];
-      seg_c[base + 32 * m] = (float)cv;
+      seg_c[slot_at<PAIR>(i, base, m)] = (float)cv;
       srow = add(srow, cv);
     }
     s32[i] = (float)srow;
@@ -356,7 +365,7 @@ __global__ void k_assex3(int nseg, int nelem, int ld, const int2 *__restrict__ s
 // the Dirichlet values scattered to their nodes, SM corrected, the rows and
 // columns of the Dirichlet nodes masked.  nbor is 1-based (MESH%NBOR).
 // NBOR entries outside 1..NPOIN are skipped and flagged in *err.
-__global__ void k_diri_scatter(int nptfr, int npoin, const int *__restrict__ nbor,
+static __global__ void k_diri_scatter(int nptfr, int npoin, const int *__restrict__ nbor,
                                const int *__restrict__ limdir, int kdir,
                                const double *__restrict__ fbor, double *w1, int *err) {
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nptfr; k += gridDim.x * blockDim.x)
@@ -371,14 +380,14 @@ __global__ void k_diri_scatter(int nptfr, int npoin, const int *__restrict__ nbo
 }
 
 // SM = SM - W2 ('X=X-Y'), then W2 = 1 ('X=C')
-__global__ void k_diri_nodes(int npoin, double *sm, double *w2) {
+static __global__ void k_diri_nodes(int npoin, double *sm, double *w2) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npoin; i += gridDim.x * blockDim.x) {
     sm[i] = sub(sm[i], w2[i]);
     w2[i] = 1.0;
   }
 }
 
-__global__ void k_diri_aux(int nptfr, int npoin, const int *__restrict__ nbor,
+static __global__ void k_diri_aux(int nptfr, int npoin, const int *__restrict__ nbor,
                            const int *__restrict__ limdir, int kdir,
                            const double *__restrict__ fbor, const double *__restrict__ dm,
                            double *sm, double *w2, double *f) {
@@ -392,7 +401,7 @@ __global__ void k_diri_aux(int nptfr, int npoin, const int *__restrict__ nbor,
     }
 }
 
-__global__ void k_diri_mask(int npoin, const double *__restrict__ mask, double *sm, double *f,
+static __global__ void k_diri_mask(int npoin, const double *__restrict__ mask, double *sm, double *f,
                             double *w2) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npoin; i += gridDim.x * blockDim.x) {
     sm[i] = mul(sm[i], mask[i]);
@@ -404,7 +413,7 @@ __global__ void k_diri_mask(int npoin, const double *__restrict__ mask, double *
 // Self-test of the bounded waits: one block enters a grid barrier one
 // arrival short (as if another block never came), so its wait must give up
 // after timeout_ns and record ST_TIMEOUT instead of hanging.
-__global__ void k_selftest_wait(Ctl *ctl, long long timeout_ns) {
+static __global__ void k_selftest_wait(Ctl *ctl, long long timeout_ns) {
   int nbar = 1;
   grid_barrier(ctl, timeout_ns, nbar);
 }
@@ -415,7 +424,7 @@ __global__ void k_selftest_wait(Ctl *ctl, long long timeout_ns) {
 // (ovd.f:92-102: |D| > 1e-10 ? 1/D : 1.0); diagonal of D.A.D
 // (om1111.f:561-570: 'Q' -> DM*D*D, 'I' -> D*D); B = B*D.
 // ---------------------------------------------------------------------------
-__global__ void k_precd1_nodes(int npoin, int precon, int td_in, const double *__restrict__ dm,
+static __global__ void k_precd1_nodes(int npoin, int precon, int td_in, const double *__restrict__ dm,
                                double *x, const double *b_in, double *b_out, double *dsc,
                                double *dms) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npoin; i += gridDim.x * blockDim.x) {
@@ -439,7 +448,7 @@ __global__ void k_precd1_nodes(int npoin, int precon, int td_in, const double *_
 // Off-diagonal part of OM1111 'M=DMD' (om1111.f:589-600):
 // XM(e,1)*D(i2)*D(i1), XM(e,2)*D(i3)*D(i1), XM(e,3)*D(i3)*D(i2) (and the
 // same for columns 4..6 of 'Q' storage).
-__global__ void k_precd1_elems(int nelem, int ndiag, const int *__restrict__ ik,
+static __global__ void k_precd1_elems(int nelem, int ndiag, const int *__restrict__ ik,
                                const double *__restrict__ dsc, const double *__restrict__ xm,
                                double *xms) {
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nelem; e += gridDim.x * blockDim.x) {
@@ -481,7 +490,7 @@ __global__ void k_build_rec(int npoin, int nelem, const int *__restrict__ ptr,
 // storage).  rec_slot holds, per record, the slots of its two neighbours.
 constexpr int MAX_NEIGHBOURS = 64;
 
-template <int TD>
+template <int TD, bool PAIR = false>
 __global__ void k_build_seg32(int npoin, int nelem, const int *__restrict__ ptr,
                               const int *__restrict__ ek, const double *__restrict__ xm,
                               const double *__restrict__ da, const int *__restrict__ meta,
@@ -504,7 +513,7 @@ __global__ void k_build_seg32(int npoin, int nelem, const int *__restrict__ ptr,
       c64[sl.y] = add(c64[sl.y], xb);
       s = add(s, add(xa, xb));
     }
-    for (int q = 0; q < nnb; ++q) seg_c[sb + 32 * q] = (float)c64[q];
+    for (int q = 0; q < nnb; ++q) seg_c[slot_at<PAIR>(i, sb, q)] = (float)c64[q];
     s32[i] = (float)s;
   }
 }
@@ -1806,7 +1815,7 @@ __global__ void __launch_bounds__(CG_THREADS, MINB) k_mixed(MixP P) {
 // ew layout: [0] mass diagonal (same for the three points), [1..3] diffusion
 // diagonal of points 1..3.
 // ---------------------------------------------------------------------------
-__global__ void k_wave_elems(int nelem, const int *__restrict__ ik, const double *__restrict__ xc,
+static __global__ void k_wave_elems(int nelem, const int *__restrict__ ik, const double *__restrict__ xc,
                              const double *__restrict__ yc, const double *__restrict__ coef,
                              double *xm, double *ew, int *err) {
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nelem; e += gridDim.x * blockDim.x) {
@@ -1905,7 +1914,7 @@ __global__ void k_mass_diff_elems(int nelem, const int *__restrict__ ik,
   }
 }
 
-__global__ void k_wave_nodes(int npoin, const int *__restrict__ ptr, const int *__restrict__ ek,
+static __global__ void k_wave_nodes(int npoin, const int *__restrict__ ptr, const int *__restrict__ ek,
                              int nelem, const double *__restrict__ ew, double *dm) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npoin; i += gridDim.x * blockDim.x) {
     double sm = 0.0, sd = 0.0;
@@ -1921,7 +1930,7 @@ __global__ void k_wave_nodes(int npoin, const int *__restrict__ ptr, const int *
 // Per-element gradient g_e = -lambda_e^T K_e x_e with K_e the unit-
 // coefficient MT02AA element matrix (rows sum to zero, so
 // lambda^T K x = -sum_{k<l} K_kl (lambda_k - lambda_l)(x_k - x_l)).
-__global__ void k_coef_grad(int nelem, const int *__restrict__ ik, const double *__restrict__ xc,
+static __global__ void k_coef_grad(int nelem, const int *__restrict__ ik, const double *__restrict__ xc,
                             const double *__restrict__ yc, const double *__restrict__ lam,
                             const double *__restrict__ xs, double *grad) {
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nelem; e += gridDim.x * blockDim.x) {

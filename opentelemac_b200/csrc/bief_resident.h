@@ -1,0 +1,109 @@
+// bief_resident.h -- the solvers that keep their search direction in shared
+// memory (bief_resident.cu), as bief_api.cu launches them.
+#pragma once
+
+#include "bief_device.cuh"
+
+namespace bief {
+
+constexpr int RES_T = 1024;      // threads of a virtual block (the tree's)
+constexpr int RES_MAXCL = 16;    // blocks of a cluster
+
+// Partition of the nodes over physical blocks, and the local index lists.
+struct ResPart {
+  int n, G, S, V, R, TP, NP;  // nodes; virtual blocks; splits; virtual blocks per block;
+                              // rows per thread; threads per block; physical blocks
+  int own;                    // V * R * TP: local indices of the block's own rows
+  const int *halo_off;        // [NP+1]
+  const int *halo;            // node numbers, ascending per block
+  const unsigned *halo_loc;   // CL: owner block << 16 | owner's local index
+};
+
+constexpr int PLAN_W = 20480;
+
+struct PlanP {
+  ResPart Q;
+  const int *meta, *seg_off, *seg_col;   // distinct neighbours (halo)
+  const int *rec_off;                    // records: meta's low half entries
+  const int2 *rec_idx;
+  const int *sg_meta, *sg_off, *sg_col;  // segment slots, when sg_li
+  int *halo_n;
+  int *halo;
+  unsigned *halo_loc;
+  unsigned short *seg_li, *sg_li, *sg_li2;  // pairs, single, pairs
+  int shift;  // pairs: 2 = indices as byte offsets into a binary32 window
+  ushort2 *rec_li;
+};
+
+struct RedShared {
+  double ws[2][32];
+  double cold[3];   // scalars of the mixed solve
+  double us[2][16];  // alternate: a warp may still read the previous reduction's
+  int err;
+};
+
+struct ResP {
+  ResPart Q;
+  Sell S;                     // operator of the storage (old-form lists for A x)
+  const unsigned short *li;   // binary32 slots / segment slots: local neighbour
+  const ushort2 *rli;         // records: local vertices
+  int td;                     // working TYPDIA
+  const double *da, *dsc;
+  double *x;
+  const double *b;
+  Ctl *ctl;
+  double *part;
+  long long timeout_ns;
+  int cache;                  // operator slots (multiple of 32) kept in shared memory
+  int halo_max;
+  int nvec;                   // own-row vectors in shared memory
+  // k_cg_res
+  int nitmax;
+  int keep;                   // steps whose slots are loaded to stay in L2
+  double eps;
+  double *r, *ad;
+  // k_mixed_res
+  int max_outer, max_inner;
+  double outer_tol, inner_tol;
+  float *z, *ri, *q;
+};
+
+// Shared-memory layout, computed alike by host and kernel.
+struct ResLayout {
+  size_t win, vec, red, box, off, deg, cidx, ccoef, total;
+};
+// elt: bytes of a vector value (8 binary64, 4 binary32); nvec: own-row
+// vectors kept beside the window; cb: operator bytes per slot without index,
+// ib: index bytes per slot.
+__host__ __device__ inline ResLayout res_layout(int own, int halo, int G, bool cl, int elt,
+                                                int nvec, int cb, int ib, int cache) {
+  ResLayout L;
+  size_t o = 0;
+  auto take = [&](size_t bytes) {
+    const size_t at = o;
+    o = (o + bytes + 15) & ~(size_t)15;
+    return at;
+  };
+  L.win = take((size_t)elt * (size_t)(own + halo));
+  L.vec = take((size_t)elt * own * nvec);
+  L.red = take(sizeof(RedShared));
+  L.box = take(cl ? (size_t)2 * 32 * G * 16 : 0);
+  L.off = take(sizeof(int2) * (size_t)(own / 32));
+  L.deg = take((size_t)own);
+  L.ccoef = take((size_t)cb * cache);
+  L.cidx = take((size_t)ib * cache);
+  L.total = o;
+  return L;
+}
+
+// Launchers (bief_resident.cu); they return cudaGetLastError()'s value.
+cudaError_t res_launch_plan(bool fill, const PlanP &A, cudaStream_t st);
+cudaError_t res_launch_cg(int sto, bool cl, const ResP &P, size_t smem, cudaStream_t st);
+// shift: 0 when the local indices are byte offsets, else 2.
+cudaError_t res_launch_mixed(int sto, bool cl, bool vs, int shift, const ResP &P, size_t smem,
+                             cudaStream_t st);
+// Whether a cluster of np blocks of tp threads with that much shared memory
+// can be resident (one probe for all cluster kernels).
+bool res_cluster_fits(int np, int tp, size_t smem);
+
+}  // namespace bief
