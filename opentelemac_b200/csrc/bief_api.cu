@@ -95,6 +95,7 @@ struct bief_handle {
   ResPart res = {};
   int res_halo_max = 0, max_deg = 0, max_sgdeg = 0, smem_max = 0;
   int *d_res_off = nullptr, *d_res_halo = nullptr;
+  unsigned long long *d_res_box = nullptr;  // tagged partial sums of the grid form
   unsigned *d_res_loc = nullptr;
   unsigned short *d_seg_li = nullptr, *d_sg_li = nullptr, *d_sg_li2 = nullptr;
   int res_shift = 0;  // binary32 local indices: 0 byte offsets, 2 element numbers
@@ -387,15 +388,26 @@ static int res_mixed_vecs(const bief_handle *h);
 // dot-product tree's shape or the segment numbering changes).
 // ---------------------------------------------------------------------------
 void res_drop(bief_handle *h) {
-  void *bufs[] = {h->d_res_off, h->d_res_halo, h->d_res_loc, h->d_seg_li, h->d_sg_li, h->d_sg_li2,
+  void *bufs[] = {h->d_res_off, h->d_res_halo, h->d_res_loc, h->d_res_box, h->d_seg_li, h->d_sg_li, h->d_sg_li2,
                   h->d_rec_li};
   for (void *p : bufs)
     if (p) cudaFree(p);
   h->d_res_off = h->d_res_halo = nullptr;
   h->d_res_loc = nullptr;
+  h->d_res_box = nullptr;
   h->d_seg_li = h->d_sg_li = h->d_sg_li2 = nullptr;
   h->d_rec_li = nullptr;
   h->res_state = 0;
+}
+
+// Tagged partial sums: 2 halves of G two-word values, cleared before each
+// launch (the tags count from 1).
+static size_t res_box_words(int G) { return G <= RES_TAG ? (size_t)4 * G : 0; }
+
+static int res_clear(bief_handle *h, cudaStream_t s) {
+  if (!h->res_cl && h->res.G <= RES_TAG)
+    CK(cudaMemsetAsync(h->d_res_box, 0, sizeof(unsigned long long) * res_box_words(h->res.G), s));
+  return BIEF_OK;
 }
 
 int res_ensure(bief_handle *h, cudaStream_t st) {
@@ -413,7 +425,7 @@ int res_ensure(bief_handle *h, cudaStream_t st) {
     const long long hi = b + 1 >= Q.G ? Q.n : (((long long)(b + 1) * Q.n / Q.G) & ~31LL);
     Q.R = std::max(Q.R, (int)((hi - lo + RES_T - 1) / RES_T));
   }
-  // Up to 16 tree blocks (32,768 nodes): one cluster, each tree block's warps
+  // Up to 8 tree blocks (16,384 nodes): one cluster, each tree block's warps
   // shared out over as many of its blocks as there are.
   h->res_cl = false;
   if (Q.G <= RES_MAXCL && Q.R <= 2) {
@@ -454,6 +466,7 @@ int res_ensure(bief_handle *h, cudaStream_t st) {
   }
   if (Q.own + most > 0xffff) return BIEF_OK;
   const bool sg = h->has_segments != 0;
+  if (!h->res_cl && (stt = dalloc(&h->d_res_box, res_box_words(Q.G)))) return stt;
   if ((stt = dalloc(&h->d_res_halo, (size_t)total)) || (stt = dalloc(&h->d_res_loc, (size_t)total)) ||
       (stt = dalloc(&h->d_seg_li, (size_t)h->nseg)) || (stt = dalloc(&h->d_rec_li, (size_t)h->nrec + 32)) ||
       (sg && ((stt = dalloc(&h->d_sg_li, (size_t)h->nsg_slots + 32)) ||
@@ -612,24 +625,21 @@ int build_transposed(bief_handle *h, const double *xm, cudaStream_t st, Sell *ou
   return BIEF_OK;
 }
 
-// GRACJG with the search direction in shared memory; *done = false when the
-// mesh's window does not fit (k_cg64 then).
-int res_cg(bief_handle *h, const CgP &C, int td, cudaStream_t s, bool *done) {
-  *done = false;
-  int st = res_ensure(h, s);
-  if (st || h->res_state != 1) return st;
-  const ResPart &Q = h->res;
-  const int cb = h->sto == 3 ? 8 : 16, ib = h->sto == 3 ? 2 : 4;
-  int nvec = h->res_cl ? 3 : 2;  // R, AD (and X) of the own rows
-  size_t base = res_layout(Q.own, h->res_halo_max, Q.G, h->res_cl, 8, nvec, cb, ib, 0).total;
-  if (base > (size_t)h->smem_max) {
-    if (h->res_cl) return BIEF_OK;
-    nvec = 0;
-    base = res_layout(Q.own, h->res_halo_max, Q.G, h->res_cl, 8, nvec, cb, ib, 0).total;
-    if (base > (size_t)h->smem_max) return BIEF_OK;
-  }
+// Steps (rows per thread) of an operator larger than the L2 whose slots are
+// loaded to stay there: 0.45 of the L2 in all, the others stream through it.
+// Measured at 1.0M nodes, 7 steps of 17 MB: 30.1 us per iteration with every
+// step streamed, 28.2 / 27.4 / 27.2 / 28.9 / 33.0 with 1 to 5 steps kept.
+static int res_keep(const bief_handle *h, bool streams, int bytes_per_slot) {
+  const int steps = h->res.V * h->res.R;
+  const double op = bytes_per_slot * (double)(h->sto == 3 ? h->nsg_slots : h->nrec);
+  return streams ? (int)(0.45 * h->l2_bytes / (op / steps)) : steps;
+}
+
+// Fields that every resident kernel takes from its solver's parameters.
+template <class CP>
+ResP res_params(const bief_handle *h, const CP &C, int td) {
   ResP P = {};
-  P.Q = Q;
+  P.Q = h->res;
   P.S = C.S;
   P.li = h->d_sg_li;
   P.rli = h->d_rec_li;
@@ -640,23 +650,37 @@ int res_cg(bief_handle *h, const CgP &C, int td, cudaStream_t s, bool *done) {
   P.b = C.b;
   P.ctl = C.ctl;
   P.part = C.part;
+  P.box = h->d_res_box;
   P.timeout_ns = C.timeout_ns;
-  P.cache = res_cache_slots(h, base, cb + ib);
   P.halo_max = h->res_halo_max;
+  return P;
+}
+
+// GRACJG with the search direction in shared memory; *done = false when the
+// mesh's window does not fit (k_cg64 then).
+int res_cg(bief_handle *h, const CgP &C, int td, cudaStream_t s, bool *done) {
+  *done = false;
+  if (h->res_state != 1) return BIEF_OK;
+  const ResPart &Q = h->res;
+  const int cb = h->sto == 3 ? 8 : 16, ib = h->sto == 3 ? 2 : 4;
+  int nvec = h->res_cl ? 3 : 2;  // R, AD (and X) of the own rows
+  auto layout = [&](int cache) {
+    return res_layout(Q.own, h->res_halo_max, Q.G, h->res_cl, 8, nvec, cb, ib, cache).total;
+  };
+  if (layout(0) > (size_t)h->smem_max) {
+    if (h->res_cl) return BIEF_OK;
+    nvec = 0;
+    if (layout(0) > (size_t)h->smem_max) return BIEF_OK;
+  }
+  ResP P = res_params(h, C, td);
+  P.cache = res_cache_slots(h, layout(0), cb + ib);
   P.nitmax = C.nitmax;
   P.nvec = nvec;
   P.eps = C.eps;
-  // An operator larger than the L2: the slots of the leading steps, 0.45 of
-  // the L2 in all, are loaded to stay there, the others stream through it
-  // (1.0M nodes, 7 steps of 17 MB: 30.1 us per iteration with every step
-  // streamed, 28.2 / 27.4 / 27.2 / 28.9 / 33.0 with 1 to 5 steps kept).
-  const double op = (cb + ib) * (double)(h->sto == 3 ? h->nsg_slots : h->nrec);
-  P.keep = C.S.cs_rec ? (int)(0.45 * h->l2_bytes / (op / (Q.V * Q.R))) : Q.V * Q.R;
+  P.keep = res_keep(h, C.S.cs_rec != 0, cb + ib);
   P.r = C.r;
   P.ad = C.ad;
-  const size_t smem =
-      res_layout(Q.own, h->res_halo_max, Q.G, h->res_cl, 8, nvec, cb, ib, P.cache).total;
-  CK(res_launch_cg(h->sto, h->res_cl, P, smem, s));
+  CK(res_launch_cg(h->sto, h->res_cl, P, layout(P.cache), s));
   h->launches++;
   *done = true;
   return BIEF_OK;
@@ -679,24 +703,11 @@ bool res_mixed_fits(const bief_handle *h) {
 }
 
 int res_mixed(bief_handle *h, const MixP &C, int td, cudaStream_t s) {
-  const ResPart &Q = h->res;
   const int nvec = res_mixed_vecs(h);
-  const size_t base = res_mixed_layout(h, nvec, 0);
-  ResP P = {};
-  P.Q = Q;
-  P.S = C.S;
+  ResP P = res_params(h, C, td);
   P.li = h->sto == 3 ? h->d_sg_li2 : h->d_seg_li;
-  P.td = td;
-  P.da = C.da;
-  P.dsc = C.dsc;
-  P.x = C.x;
-  P.b = C.b;
-  P.ctl = C.ctl;
-  P.part = C.part;
-  P.timeout_ns = C.timeout_ns;
-  P.cache = res_cache_slots(h, base, 6) / 64 * 64;
+  P.cache = res_cache_slots(h, res_mixed_layout(h, nvec, 0), 6) / 64 * 64;
   P.nvec = nvec;
-  P.halo_max = h->res_halo_max;
   P.max_outer = C.max_outer;
   P.max_inner = C.max_inner;
   P.outer_tol = C.outer_tol;
@@ -1274,6 +1285,7 @@ int bief_solve_dev(bief_handle *h, double *x, double *b, bief_slvcfg *cfg, int f
     P.timeout_ns = h->timeout_ns;
     bool done = false;
     if (!comp && (st = res_ensure(h, s))) return st;  // plan outside the timed launch
+    if (!comp && h->res_state == 1 && (st = res_clear(h, s))) return st;
     CK(cudaEventRecord(h->ev[0], s));
     if (!comp && (st = res_cg(h, P, td, s, &done))) return st;
     if (!done && (st = launch_coop(h, cg_kernel(td, h->sto, comp, h->wide), &P, s))) return st;
@@ -1380,6 +1392,7 @@ int bief_solve_mixed_dev(bief_handle *h, double *x, const double *b, int precon,
   P.ctl = h->d_ctl;
   P.timeout_ns = h->timeout_ns;
   CK(cudaMemsetAsync(h->d_ctl, 0, sizeof(Ctl), s));
+  if (pair && (st = res_clear(h, s))) return st;
   CK(cudaEventRecord(h->ev[0], s));
   if ((st = pair ? res_mixed(h, P, td, s)
                  : launch_coop(h, mixed_kernel(td, h->sto, h->wide, slots16(h)), &P, s)))

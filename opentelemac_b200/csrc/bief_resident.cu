@@ -268,44 +268,77 @@ __device__ __forceinline__ T warp_tree(T v) {
   return v;
 }
 
+// A value with the number of its reduction beside each 32 bits of it: one or
+// two 64-bit words, each valid as soon as it shows the number waited for.
+template <typename T>
+__device__ __forceinline__ void tag_words(T u, unsigned tag, unsigned long long &x,
+                                          unsigned long long &y) {
+  if constexpr (sizeof(T) == 8) {
+    const unsigned long long bits = (unsigned long long)__double_as_longlong((double)u);
+    x = (bits << 32) | tag;
+    y = (bits & 0xffffffff00000000ull) | tag;
+  } else {
+    x = ((unsigned long long)__float_as_uint((float)u) << 32) | tag;
+    y = tag;
+  }
+}
+template <typename T>
+__device__ __forceinline__ T tag_value(unsigned long long x, unsigned long long y) {
+  if constexpr (sizeof(T) == 8)
+    return __longlong_as_double((long long)((x >> 32) | (y & 0xffffffff00000000ull)));
+  else
+    return __uint_as_float((unsigned)(x >> 32));
+}
+
+// How the blocks of a solve talk to each other.
+//   COM_CL   cluster: every warp's total goes straight to every block's shared
+//            memory as tagged words, halo values are read from there;
+//   COM_TAG  grid: block totals as tagged words that all blocks poll;
+//   COM_CNT  grid: block totals and an arrival counter.
+// Measured per reduction in a loop of nothing else at 1024 threads (us):
+// counter 2.5 (1 to 75 blocks) to 2.6 (148); tagged, without / with fences,
+// 17 blocks 1.1 / 1.6, 44 blocks 2.5 / 2.5, 148 blocks 5.5 / 5.3, as polls
+// queue at an L2 line and delay the write they wait for.  So tags up to
+// RES_TAG blocks (23k nodes, 10 blocks: 8.7 against 10.2 us per iteration).
+//
+// PUB: the reduction also publishes what the block wrote before it (R for
+// its neighbours' halos).  Without it tagged words need no fence: what the
+// block read before is already in the partial sums it sends.
+enum : int { COM_CL = 0, COM_TAG = 1, COM_CNT = 2 };
+
 // Communication state of one block.
-template <bool CL>
+template <int COM>
 struct Comm {
+  static constexpr bool CL = COM == COM_CL;
   Ctl *ctl;
   double *part;               // grid form: 2 halves of G partials
   long long timeout_ns;
   RedShared *sh;
-  unsigned long long *box;    // cluster form: 2 halves of 32 G tagged words (16 B each)
+  unsigned long long *box;    // tagged words, 2 halves: cluster 32 G (shared memory), grid G
   int G, V, S, NP, p;
-  unsigned nbar;
+  unsigned nbar;              // reductions so far
+
+  // a publishing reduction made on a copy of this state
+  __device__ __forceinline__ void done() { ++nbar; }
 
   // v: this thread's partial per virtual block of the block (V of them).
-  // All writes of this block made before are visible to whoever returns from
-  // the matching wait().
-  template <typename T>
+  template <bool PUB, typename T>
   __device__ __forceinline__ void send(const T *v) {
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    unsigned long long x, y;
     ++nbar;
     if constexpr (CL) {
-      // every warp's total goes to every block of the cluster: lane c writes
-      // it, with the reduction's number beside each 32 bits, to block c
       const T u = warp_tree(v[0]);
-      __syncwarp();
-      fence_cluster();
+      if (PUB) {
+        __syncwarp();
+        fence_cluster();
+      }
       if (lane < NP) {
         const int vw = (p % S) * ((int)blockDim.x >> 5) + w;
         const int slot = (p / S) * 32 + vw;
         const unsigned a =
             mapa(smem_addr(box + 2 * ((size_t)(nbar & 1) * 32 * G + slot)), (unsigned)lane);
-        unsigned long long x, y;
-        if constexpr (sizeof(T) == 8) {
-          const unsigned long long bits = (unsigned long long)__double_as_longlong((double)u);
-          x = (bits << 32) | nbar;
-          y = (bits & 0xffffffff00000000ull) | nbar;
-        } else {
-          x = ((unsigned long long)__float_as_uint((float)u) << 32) | nbar;
-          y = nbar;
-        }
+        tag_words(u, nbar, x, y);
         asm volatile("st.relaxed.cluster.shared::cluster.v2.b64 [%0], {%1, %2};" ::"r"(a), "l"(x),
                      "l"(y)
                      : "memory");
@@ -318,13 +351,24 @@ struct Comm {
       }
       __syncthreads();
       if (w == 0) {
-        double *buf = part + (size_t)(nbar & 1) * G;
+        if (PUB && COM == COM_TAG) fence_gpu();
 #pragma unroll 1
         for (int q = 0; q < V; ++q) {
           const T u = warp_tree((T)sh->ws[q][lane]);
-          if (lane == 0 && p * V + q < G) buf[p * V + q] = (double)u;
+          const int b = p * V + q;
+          if (b >= G) break;
+          if (lane) continue;
+          if constexpr (COM == COM_TAG) {
+            tag_words(u, nbar, x, y);
+            asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(
+                             box + 2 * ((size_t)(nbar & 1) * G + b)),
+                         "l"(x), "l"(y)
+                         : "memory");
+          } else {
+            part[(size_t)(nbar & 1) * G + b] = (double)u;
+          }
         }
-        if (lane == 0)
+        if (COM == COM_CNT && lane == 0)
           asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&ctl->arrivals), "l"(1ull)
                        : "memory");
       }
@@ -332,34 +376,46 @@ struct Comm {
   }
 
   // The sum over all blocks; false when the bounded wait ran out.
-  template <typename T>
+  template <bool PUB, typename T>
   __device__ __forceinline__ bool wait(T &out) {
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    int ns;
-    if constexpr (CL) {
-      ns = G;
-      int bad = 0;
-      if (w < G) {  // warp w: the 32 warp totals of virtual block w
-        const unsigned a = smem_addr(box + 2 * ((size_t)(nbar & 1) * 32 * G + t));
-        unsigned long long x, y, t0 = 0;
+    int ns, bad = 0;
+    if constexpr (COM != COM_CNT) {
+      // cluster: warp w sums the 32 warp totals of virtual block w; grid: the
+      // totals of virtual blocks 32 w ..
+      ns = CL ? G : (G + 31) >> 5;
+      if (w < ns) {
+        T u = T(0);
+        if (CL || t < G) {
+          const unsigned long long *m =
+              box + 2 * ((size_t)(nbar & 1) * (CL ? 32 : 1) * G + t);
+          unsigned long long x, y, t0 = 0;
 #pragma unroll 1
-        for (unsigned n = 1;; ++n) {
-          asm volatile("ld.relaxed.cluster.shared::cta.v2.b64 {%0, %1}, [%2];"
-                       : "=l"(x), "=l"(y)
-                       : "r"(a)
-                       : "memory");
-          if ((unsigned)x == nbar && (unsigned)y == nbar) break;
-          if ((n & 0xfff) == 0) {
-            if (!t0) t0 = global_ns();
-            else if ((long long)(global_ns() - t0) > timeout_ns) { bad = 1; break; }
+          for (unsigned n = 1;; ++n) {
+            if constexpr (CL)
+              asm volatile("ld.relaxed.cluster.shared::cta.v2.b64 {%0, %1}, [%2];"
+                           : "=l"(x), "=l"(y)
+                           : "r"(smem_addr(m))
+                           : "memory");
+            else
+              asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];"
+                           : "=l"(x), "=l"(y)
+                           : "l"(m)
+                           : "memory");
+            if ((unsigned)x == nbar && (unsigned)y == nbar) break;
+            if ((n & 0xff) == 0) {
+              if (!t0) t0 = global_ns();
+              else if ((long long)(global_ns() - t0) > timeout_ns) { bad = 1; break; }
+            }
           }
+          u = tag_value<T>(x, y);
+          if (!CL) u = add(T(0), u);
         }
-        fence_cluster();
-        T u;
-        if constexpr (sizeof(T) == 8)
-          u = __longlong_as_double((long long)((x >> 32) | (y & 0xffffffff00000000ull)));
-        else
-          u = __uint_as_float((unsigned)(x >> 32));
+        if (PUB) {
+          if (CL) fence_cluster();
+          else fence_gpu();
+        }
+        __syncwarp();
         u = warp_tree(u);
         if (lane == 0) reinterpret_cast<T *>(sh->us[nbar & 1])[w] = u;
       }
@@ -371,7 +427,6 @@ struct Comm {
       if (t == 0) {
         const unsigned long long target = (unsigned long long)nbar * (unsigned long long)NP;
         unsigned long long t0 = 0, c;
-        int e = 0;
 #pragma unroll 1
         for (unsigned n = 1;; ++n) {
           asm volatile("ld.acquire.gpu.global.u64 %0, [%1];"
@@ -382,16 +437,14 @@ struct Comm {
           if ((n & 0xff) == 0) {
             if (!t0) t0 = global_ns();
             else if ((long long)(global_ns() - t0) > timeout_ns) {
-              e = 1;
+              bad = 1;
               atomicExch(&ctl->status, (int)ST_TIMEOUT);
               break;
             }
           }
         }
-        sh->err = e;
       }
-      __syncthreads();
-      if (sh->err) return false;
+      if (__syncthreads_or(bad)) return false;
       ns = (G + 31) >> 5;
       if (w < ns) {
         const double *buf = part + (size_t)(nbar & 1) * G;
@@ -757,28 +810,28 @@ struct Halo {
 };
 
 // A reduction off the iteration's path (one copy of the code per type).
-template <bool CL, typename T>
-__device__ __noinline__ bool cold_reduce(Comm<CL> M, T v0, T v1, T *out) {
+template <int COM, typename T>
+__device__ __noinline__ bool cold_reduce(Comm<COM> M, T v0, T v1, T *out) {  // the caller counts it: done()
   const T v[2] = {v0, v1};
-  M.send(v);
-  return M.wait(*out);
+  M.template send<true>(v);
+  return M.template wait<true>(*out);
 }
 
-template <bool CL>
-__device__ __forceinline__ void comm_init(Comm<CL> &M, const ResP &P, int V, unsigned char *red,
+template <int COM>
+__device__ __forceinline__ void comm_init(Comm<COM> &M, const ResP &P, int V, unsigned char *red,
                                           unsigned char *box) {
   M.ctl = P.ctl;
   M.part = P.part;
   M.timeout_ns = P.timeout_ns;
   M.sh = reinterpret_cast<RedShared *>(red);
-  M.box = reinterpret_cast<unsigned long long *>(box);
+  M.box = COM == COM_CL ? reinterpret_cast<unsigned long long *>(box) : P.box;
   M.G = P.Q.G;
   M.V = V;
   M.S = P.Q.S;
   M.NP = P.Q.NP;
   M.p = blockIdx.x;
   M.nbar = 0;
-  if (CL)
+  if (COM == COM_CL)
 #pragma unroll 1
     for (int i = threadIdx.x; i < 2 * 32 * M.G * 2; i += blockDim.x) M.box[i] = 0;
 }
@@ -792,8 +845,9 @@ __device__ __forceinline__ void comm_init(Comm<CL> &M, const ResP &P, int V, uns
 // the loop outgrew the instruction caches, and with most of the SM's memory
 // taken as shared memory every register spill is an L2 access.
 // ---------------------------------------------------------------------------
-template <int STO, bool CL, int MT>
+template <int STO, int COM, int MT>
 __global__ void __launch_bounds__(MT, 1) k_cg_res(const __grid_constant__ ResP P) {
+  constexpr bool CL = COM == COM_CL;
   using ROW = typename std::conditional<STO == 3, SegRow, RecRow>::type;
   using C = typename ROW::C;
   using I = typename ROW::I;
@@ -819,7 +873,7 @@ __global__ void __launch_bounds__(MT, 1) k_cg_res(const __grid_constant__ ResP P
     gc = P.S.rec_c;
     gi = reinterpret_cast<const unsigned *>(P.rli);
   }
-  Comm<CL> M;
+  Comm<COM> M;
   comm_init(M, P, V, res_sm + L.red, res_sm + L.box);
   res_setup<C, I, 1>(Q, p, P.S.meta, 0, P.S.rec_off, gc, gi, P.cache, s_off, s_deg, s_c, s_i);
   if constexpr (CL) cluster_sync();  // every block of the cluster has cleared its box
@@ -884,8 +938,8 @@ __global__ void __launch_bounds__(MT, 1) k_cg_res(const __grid_constant__ ResP P
     double xl;
     {
       double got;
-      if (!cold_reduce<CL, double>(M, s[0], s[1], &got)) return;
-      ++M.nbar;
+      if (!cold_reduce<COM, double>(M, s[0], s[1], &got)) return;
+      M.done();
       xl = got;
     }
     int relat = 1, m = 0, phase = 0, status = ST_OK;
@@ -940,8 +994,20 @@ __global__ void __launch_bounds__(MT, 1) k_cg_res(const __grid_constant__ ResP P
         else P.ad[i] = acc;
         dacc(v, d0, acc);
       });
-      M.send(s);
-      if (!M.wait(red)) return;
+      // the first product's residual is published (the counter always does;
+      // one reduction for every phase, as a call here costs the loop registers)
+      if constexpr (COM == COM_CNT) {
+        M.template send<true>(s);
+        if (!M.template wait<true>(red)) return;
+      } else if (phase == 0) {
+        double got;
+        if (!cold_reduce<COM, double>(M, s[0], s[1], &got)) return;
+        M.done();
+        red = got;
+      } else {
+        M.template send<false>(s);
+        if (!M.template wait<false>(red)) return;
+      }
       if (phase == 0) {
         rmrm = rmgm = red;
         if (isnan(rmrm)) { status = ST_NAN; break; }
@@ -963,7 +1029,7 @@ __global__ void __launch_bounds__(MT, 1) k_cg_res(const __grid_constant__ ResP P
           put_r(a, i, ri);
           dacc(v, ri, ri);
         });
-        M.send(s);
+        M.template send<true>(s);
       }
       // X = X - RO*D (:268 / :387) while the partial sums travel
       if constexpr (CL) {
@@ -987,7 +1053,7 @@ __global__ void __launch_bounds__(MT, 1) k_cg_res(const __grid_constant__ ResP P
         }
       }
       if (stop) { status = m; break; }
-      if (!M.wait(red)) return;
+      if (!M.template wait<true>(red)) return;
       const double rm1gm1 = rmgm;
       rmrm = red;
       rmgm = rmrm;
@@ -1047,8 +1113,9 @@ __device__ __noinline__ ResidualSums mixed_residual(const ResP &P, float *s_r) {
 // own rows and their row sums in shared memory (always in the cluster form);
 // else in global memory.  SH = 0: local indices as byte offsets.
 // ---------------------------------------------------------------------------
-template <int STO, bool CL, bool VS, int SH, int MT>
+template <int STO, int COM, bool VS, int SH, int MT>
 __global__ void __launch_bounds__(MT, 1) k_mixed_res(const __grid_constant__ ResP P) {
+  constexpr bool CL = COM == COM_CL;
   extern __shared__ __align__(16) unsigned char res_sm[];
   const ResPart &Q = P.Q;
   const int t = threadIdx.x, TP = blockDim.x, lane = t & 31;
@@ -1063,7 +1130,7 @@ __global__ void __launch_bounds__(MT, 1) k_mixed_res(const __grid_constant__ Res
   unsigned *s_i = reinterpret_cast<unsigned *>(res_sm + L.cidx);
   const float2 *gc = reinterpret_cast<const float2 *>(P.S.seg_c);
   const unsigned *gi = reinterpret_cast<const unsigned *>(P.li);
-  Comm<CL> M;
+  Comm<COM> M;
   comm_init(M, P, V, res_sm + L.red, res_sm + L.box);
   res_setup<float2, unsigned, 2>(Q, p, P.S.meta, 16, P.S.seg_off, gc, gi, P.cache, s_off, s_deg,
                                  s_c, s_i);
@@ -1117,8 +1184,8 @@ __global__ void __launch_bounds__(MT, 1) k_mixed_res(const __grid_constant__ Res
           P.z[i] = 0.0f;
         }
       });
-      if (!cold_reduce<CL, double>(M, sd[0], sd[1], &got)) return;
-      ++M.nbar;
+      if (!cold_reduce<COM, double>(M, sd[0], sd[1], &got)) return;
+      M.done();
       xl = got;
     }
     if (__dsqrt_rn(xl) < 1.0e-15) {
@@ -1142,10 +1209,10 @@ __global__ void __launch_bounds__(MT, 1) k_mixed_res(const __grid_constant__ Res
       double got64;
       float got32;
       const ResidualSums sum = mixed_residual<STO, CL, VS>(P, s_r);
-      if (!cold_reduce<CL, double>(M, sum.d0, sum.d1, &got64)) return;
-      ++M.nbar;
-      if (!cold_reduce<CL, float>(M, sum.f0, sum.f1, &got32)) return;
-      ++M.nbar;
+      if (!cold_reduce<COM, double>(M, sum.d0, sum.d1, &got64)) return;
+      M.done();
+      if (!cold_reduce<COM, float>(M, sum.f0, sum.f1, &got32)) return;
+      M.done();
       const double rr = got64;
       rho = got32;
       if (t == 0) cold[2] = rr;
@@ -1219,8 +1286,8 @@ __global__ void __launch_bounds__(MT, 1) k_mixed_res(const __grid_constant__ Res
         }
       }
       float pq;
-      M.send(sf);
-      if (!M.wait(pq)) return;
+      M.template send<false>(sf);
+      if (!M.template wait<false>(pq)) return;
       if (!(pq > 0.0f)) {
         finish(isnan(pq) ? ST_NAN : ST_BREAKDOWN, cold[2], cold[0]);
         return;
@@ -1263,7 +1330,7 @@ __global__ void __launch_bounds__(MT, 1) k_mixed_res(const __grid_constant__ Res
           }
         }
       }
-      M.send(sf);
+      M.template send<true>(sf);
       if constexpr (VS) {
         rows([&](int, int a, int) { s_z[a] = add(s_z[a], mul(alpha, win[a])); });
       } else {
@@ -1286,7 +1353,7 @@ __global__ void __launch_bounds__(MT, 1) k_mixed_res(const __grid_constant__ Res
         }
       }
       rho_old = rho;
-      if (!M.wait(rho_rec)) return;
+      if (!M.template wait<true>(rho_rec)) return;
       rho = rho_rec;
       ++inner;
       last = inner >= P.max_inner;
@@ -1304,8 +1371,8 @@ __global__ void __launch_bounds__(MT, 1) k_mixed_res(const __grid_constant__ Res
       });
       if (CL) fence_gpu();  // x is read at neighbours through global memory
       float dummy;
-      if (!cold_reduce<CL, float>(M, 0.0f, 0.0f, &dummy)) return;
-      ++M.nbar;
+      if (!cold_reduce<COM, float>(M, 0.0f, 0.0f, &dummy)) return;
+      M.done();
       if (CL) fence_gpu();
     }
   };
@@ -1363,15 +1430,25 @@ cudaError_t res_launch_plan(bool fill, const PlanP &A, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+template <int STO>
+static cudaError_t launch_cg(bool cl, const ResP &P, size_t smem, cudaStream_t st) {
+  if (cl)
+    return P.Q.TP <= RES_T / 2 ? launch(k_cg_res<STO, COM_CL, RES_T / 2>, cl, P, smem, st)
+                               : launch(k_cg_res<STO, COM_CL, RES_T>, cl, P, smem, st);
+  return P.Q.G <= RES_TAG ? launch(k_cg_res<STO, COM_TAG, RES_T>, cl, P, smem, st)
+                          : launch(k_cg_res<STO, COM_CNT, RES_T>, cl, P, smem, st);
+}
+
 cudaError_t res_launch_cg(int sto, bool cl, const ResP &P, size_t smem, cudaStream_t st) {
-  const bool half = P.Q.TP <= RES_T / 2;
-  if (sto == 3)
-    return !cl    ? launch(k_cg_res<3, false, RES_T>, cl, P, smem, st)
-           : half ? launch(k_cg_res<3, true, RES_T / 2>, cl, P, smem, st)
-                  : launch(k_cg_res<3, true, RES_T>, cl, P, smem, st);
-  return !cl    ? launch(k_cg_res<1, false, RES_T>, cl, P, smem, st)
-         : half ? launch(k_cg_res<1, true, RES_T / 2>, cl, P, smem, st)
-                : launch(k_cg_res<1, true, RES_T>, cl, P, smem, st);
+  return sto == 3 ? launch_cg<3>(cl, P, smem, st) : launch_cg<1>(cl, P, smem, st);
+}
+
+template <int STO, int COM>
+static cudaError_t launch_mixed_grid(bool vs, int shift, const ResP &P, size_t smem,
+                                     cudaStream_t st) {
+  if (!vs) return launch(k_mixed_res<STO, COM, false, 2, RES_T>, false, P, smem, st);
+  return shift ? launch(k_mixed_res<STO, COM, true, 2, RES_T>, false, P, smem, st)
+               : launch(k_mixed_res<STO, COM, true, 0, RES_T>, false, P, smem, st);
 }
 
 template <int STO>
@@ -1379,11 +1456,11 @@ static cudaError_t launch_mixed(bool cl, bool vs, int shift, const ResP &P, size
                                 cudaStream_t st) {
   if (cl)
     return P.Q.TP <= RES_T / 2
-               ? launch(k_mixed_res<STO, true, true, 0, RES_T / 2>, cl, P, smem, st)
-               : launch(k_mixed_res<STO, true, true, 0, RES_T>, cl, P, smem, st);
-  if (!vs) return launch(k_mixed_res<STO, false, false, 2, RES_T>, cl, P, smem, st);
-  return shift ? launch(k_mixed_res<STO, false, true, 2, RES_T>, cl, P, smem, st)
-               : launch(k_mixed_res<STO, false, true, 0, RES_T>, cl, P, smem, st);
+               ? launch(k_mixed_res<STO, COM_CL, true, 0, RES_T / 2>, cl, P, smem, st)
+               : launch(k_mixed_res<STO, COM_CL, true, 0, RES_T>, cl, P, smem, st);
+  // (vectors in global memory: meshes of far more than RES_TAG blocks)
+  return vs && P.Q.G <= RES_TAG ? launch_mixed_grid<STO, COM_TAG>(vs, shift, P, smem, st)
+                                : launch_mixed_grid<STO, COM_CNT>(vs, shift, P, smem, st);
 }
 
 cudaError_t res_launch_mixed(int sto, bool cl, bool vs, int shift, const ResP &P, size_t smem,
@@ -1393,7 +1470,7 @@ cudaError_t res_launch_mixed(int sto, bool cl, bool vs, int shift, const ResP &P
 }
 
 bool res_cluster_fits(int np, int tp, size_t smem) {
-  auto k = k_cg_res<1, true, RES_T>;
+  auto k = k_cg_res<1, COM_CL, RES_T>;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
           cudaSuccess ||
       cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
