@@ -686,6 +686,33 @@ int res_cg(bief_handle *h, const CgP &C, int td, cudaStream_t s, bool *done) {
   return BIEF_OK;
 }
 
+// CGSTAB likewise, in the grid form with one tree block per physical block
+// and four vectors of the window in shared memory.
+int res_cgstab(bief_handle *h, const StabP &C, int td, bool comp, cudaStream_t s, bool *done) {
+  *done = false;
+  if (h->res_state != 1 || h->res_cl || h->res.V != 1) return BIEF_OK;
+  const ResPart &Q = h->res;
+  const int cb = h->sto == 3 ? 8 : 16, ib = h->sto == 3 ? 2 : 4;
+  auto layout = [&](int cache) {
+    return res_layout(Q.own, h->res_halo_max, Q.G, false, 32, 0, cb, ib, cache).total;
+  };
+  const size_t fixed = 4096;  // grid_reduce's own shared memory (under 2 KB)
+  if (layout(0) + fixed > (size_t)h->smem_max) return BIEF_OK;
+  ResP P = res_params(h, C, td);
+  P.cache = res_cache_slots(h, layout(0) + fixed, cb + ib);
+  P.nitmax = C.nitmax;
+  P.eps = C.eps;
+  P.keep = res_keep(h, C.S.cs_rec != 0, cb + ib);
+  P.r = C.r;
+  P.ad = C.v0;
+  P.tv = C.t;
+  P.p0 = C.p;
+  CK(res_launch_cgstab(h->sto, comp, P, layout(P.cache), s));
+  h->launches++;
+  *done = true;
+  return BIEF_OK;
+}
+
 // The mixed-precision solve likewise: r, q, z and the row sums of the own
 // rows in shared memory when they fit (always in the cluster form), else in
 // global memory.
@@ -1177,8 +1204,11 @@ int bief_solve_dev(bief_handle *h, double *x, double *b, bief_slvcfg *cfg, int f
     P.part = h->d_part;
     P.ctl = h->d_ctl;
     P.timeout_ns = h->timeout_ns;
+    bool done = false;
+    if ((st = res_ensure(h, s))) return st;  // plan outside the timed launch
     CK(cudaEventRecord(h->ev[0], s));
-    if ((st = launch_coop(h, cgstab_kernel(td, h->sto, comp, h->wide), &P, s))) return st;
+    if ((st = res_cgstab(h, P, td, comp, s, &done))) return st;
+    if (!done && (st = launch_coop(h, cgstab_kernel(td, h->sto, comp, h->wide), &P, s))) return st;
   } else if (cfg->slv == 7) {  // GMRES
     if (!h->d_gpart && (st = dalloc(&h->d_gpart, 4 * (size_t)h->G * (GM_MAXK + 1) + 4)))
       return st;

@@ -1067,6 +1067,174 @@ __global__ void __launch_bounds__(MT, 1) k_cg_res(const __grid_constant__ ResP P
   if constexpr (CL) cluster_sync();  // nobody leaves while another may reach its memory
 }
 
+// ---------------------------------------------------------------------------
+// CGSTAB (cgstab.f:95-200), statement for statement k_cgstab, in the grid
+// form with one tree block per physical block.  Q, S, R and V of the block's
+// nodes and of its halo are in shared memory: the halo's copies follow by
+// their owners' operations from one value per product (V, then T), where
+// k_cgstab gathered three vectors per neighbour for A Q and two for A S.
+// ---------------------------------------------------------------------------
+template <int STO, bool COMP>
+__global__ void __launch_bounds__(RES_T, 1) k_cgstab_res(const __grid_constant__ ResP P) {
+  using ROW = typename std::conditional<STO == 3, SegRow, RecRow>::type;
+  using C = typename ROW::C;
+  using I = typename ROW::I;
+  extern __shared__ __align__(16) unsigned char res_sm[];
+  const ResPart &Q = P.Q;
+  const int t = threadIdx.x, TP = RES_T, lane = t & 31, p = blockIdx.x;
+  const ResLayout L = res_layout(Q.own, P.halo_max, Q.G, false, 32, 0, sizeof(C), sizeof(I),
+                                 P.cache);
+  const int W = Q.own + P.halo_max;
+  double *wq = reinterpret_cast<double *>(res_sm + L.win), *ws = wq + W, *wr = ws + W, *wv = wr + W;
+  int2 *s_off = reinterpret_cast<int2 *>(res_sm + L.off);
+  unsigned char *s_deg = res_sm + L.deg;
+  C *s_c = reinterpret_cast<C *>(res_sm + L.ccoef);
+  I *s_i = reinterpret_cast<I *>(res_sm + L.cidx);
+  const C *gc;
+  const I *gi;
+  if constexpr (STO == 3) {
+    gc = P.S.sg_c;
+    gi = P.li;
+  } else {
+    gc = P.S.rec_c;
+    gi = reinterpret_cast<const unsigned *>(P.rli);
+  }
+  res_setup<C, I, 1>(Q, p, P.S.meta, 0, P.S.rec_off, gc, gi, P.cache, s_off, s_deg, s_c, s_i);
+  const unsigned long long pol_keep = l2_policy(false), pol_stream = l2_policy(true);
+  const int lo = (int)blk_lo(p, Q.n, Q.G) + t, hi = (int)blk_lo(p + 1, Q.n, Q.G);
+  const int h0 = Q.halo_off[p], nh = Q.halo_off[p + 1] - h0;
+  DotAcc<COMP, 2> sd;
+  double rd[2];
+  int nbar = 0;
+
+  auto rows = [&](auto f) {
+    int a = t;
+#pragma unroll 1
+    for (int i = lo; i < hi; i += RES_T, a += TP) f(a, i);
+  };
+  // f(window index, node) over the halo
+  auto halo = [&](auto f) {
+#pragma unroll 1
+    for (int h = t; h < nh; h += TP) f(Q.own + h, __ldg(Q.halo + h0 + h));
+  };
+  auto finish = [&](int status, int m, double rmrm, double xl, int relat) {
+    if (P.dsc) rows([&](int, int i) { P.x[i] = mul(P.x[i], P.dsc[i]); });  // solve.f:637-641
+    if (p == 0 && t == 0) {
+      set_status(P.ctl, status);
+      P.ctl->nit = m;
+      P.ctl->relres = __dsqrt_rn(__ddiv_rn(rmrm, xl));
+      P.ctl->relat = relat;
+    }
+  };
+
+  // XL (:105-111); SQRT(XL) < RMIN: X = 0 (:112-116)
+  sd.zero();
+  rows([&](int, int i) { sd.acc(0, P.b[i], P.b[i]); });
+  if (!dred<COMP, 2>(P.ctl, P.part, P.timeout_ns, nbar, sd, rd)) return;
+  double xl = rd[0];
+  int relat = 1;
+  if (xl < 1.0) { xl = 1.0; relat = 0; }
+  if (__dsqrt_rn(xl) < 1.0e-15) {
+    rows([&](int, int i) { P.x[i] = 0.0; });
+    finish(ST_OK, 0, 0.0, xl, relat);
+    return;
+  }
+  const double tol = mul(xl, mul(P.eps, P.eps));
+  rows([&](int a, int i) { wq[a] = P.x[i]; });
+  halo([&](int a, int j) { wq[a] = P.x[j]; });
+  double rmrm = 0.0, beta1 = 0.0, alfa = 1.0, beta = 1.0, omeg1 = 1.0;
+  int m = 0, phase = 0;
+#pragma unroll 1
+  for (;;) {
+    // phase 0: R = B - A X (:120-123); 1: V = A Q, P.V (:163, :173);
+    // phase 2: T = A S, T.S and T.T (:177, :186-187)
+    const double *win = phase == 2 ? ws : wq;
+    __syncthreads();
+    sd.zero();
+    {
+      int a = t, k = 0;
+#pragma unroll 1
+      for (int i = lo; i - lane < hi; i += RES_T, a += TP, ++k) {
+        const bool has = i < hi;
+        const double d0 = has ? win[a] : 0.0;
+        const double acc =
+            res_row<ROW>(has ? td_term(P.td, d0, P.da, i) : 0.0, s_off[a >> 5], s_deg[a], gc, gi,
+                         k < P.keep ? pol_keep : pol_stream, s_c, s_i, win);
+        if (!has) continue;
+        if (phase == 0) {
+          const double r0 = sub(P.b[i], acc);
+          wr[a] = r0;
+          __stcg(P.r + i, r0);
+          P.p0[i] = r0;
+          sd.acc(0, r0, r0);
+        } else if (phase == 1) {
+          wv[a] = acc;
+          __stcg(P.ad + i, acc);
+          sd.acc(0, P.p0[i], acc);
+        } else {
+          __stcg(P.tv + i, acc);
+          sd.acc(0, acc, d0);
+          sd.acc(1, acc, acc);
+        }
+      }
+    }
+    if (!dred<COMP, 2>(P.ctl, P.part, P.timeout_ns, nbar, sd, rd)) return;
+    if (phase == 1) {
+      omeg1 = __ddiv_rn(beta1, rd[0]);  // :174
+      const double nomeg1 = -omeg1;     // S = R - OMEG1 V (:176)
+      halo([&](int a, int j) {
+        const double v = __ldcg(P.ad + j);
+        wv[a] = v;
+        ws[a] = add(wr[a], mul(nomeg1, v));
+      });
+      rows([&](int a, int) { ws[a] = add(wr[a], mul(nomeg1, wv[a])); });
+      phase = 2;
+      continue;
+    }
+    if (phase == 2) {
+      alfa = __ddiv_rn(rd[0], rd[1]);  // :188
+      // X = X + OMEG1 Q + ALFA S (:190-191), R = S - ALFA T (:192), R.R and R.P
+      const double nalfa = -alfa;
+      sd.zero();
+      rows([&](int a, int i) {
+        const double si = ws[a];
+        P.x[i] = add(add(P.x[i], mul(omeg1, wq[a])), mul(alfa, si));
+        const double ri = add(si, mul(nalfa, __ldcg(P.tv + i)));
+        wr[a] = ri;
+        sd.acc(0, ri, ri);
+        sd.acc(1, ri, P.p0[i]);
+      });
+      halo([&](int a, int j) { wr[a] = add(ws[a], mul(nalfa, __ldcg(P.tv + j))); });
+      if (!dred<COMP, 2>(P.ctl, P.part, P.timeout_ns, nbar, sd, rd)) return;
+      rmrm = rd[0];
+      beta1 = rd[1];
+      if (isnan(rmrm)) { finish(ST_NAN, m, rmrm, xl, relat); return; }
+      if (rmrm <= tol) { finish(ST_OK, m, rmrm, xl, relat); return; }  // :194
+      if (m >= P.nitmax) { finish(m, m, rmrm, xl, relat); return; }
+    } else {
+      rmrm = rd[0];
+      if (isnan(rmrm)) { finish(ST_NAN, 0, rmrm, xl, relat); return; }
+      if (rmrm < mul(mul(P.eps, P.eps), xl)) { finish(ST_OK, 0, rmrm, xl, relat); return; }
+      beta1 = rmrm;  // R.P with P a copy of R: the same products and sum
+      // V = Q = 0 (:144-147)
+      rows([&](int a, int) { wq[a] = wv[a] = 0.0; });
+      halo([&](int a, int j) {
+        wq[a] = wv[a] = 0.0;
+        wr[a] = __ldcg(P.r + j);
+      });
+    }
+    ++m;
+    const double omeg2 = __ddiv_rn(mul(omeg1, beta1), beta);  // :156
+    const double omeg = __ddiv_rn(omeg2, alfa);
+    beta = beta1;
+    const double nomeg2 = -omeg2;
+    // Q = R + OMEG Q - OMEG2 V (:161-162)
+    rows([&](int a, int) { wq[a] = add(add(wr[a], mul(omeg, wq[a])), mul(nomeg2, wv[a])); });
+    halo([&](int a, int) { wq[a] = add(add(wr[a], mul(omeg, wq[a])), mul(nomeg2, wv[a])); });
+    phase = 1;
+  }
+}
+
 // True residual of the mixed solve, r = b - A x in binary64, r32 = (float)r
 // (to shared memory in the cluster form, else to ri; VS: both), with the
 // thread's partial sums of r.r in both precisions.
@@ -1441,6 +1609,14 @@ static cudaError_t launch_cg(bool cl, const ResP &P, size_t smem, cudaStream_t s
 
 cudaError_t res_launch_cg(int sto, bool cl, const ResP &P, size_t smem, cudaStream_t st) {
   return sto == 3 ? launch_cg<3>(cl, P, smem, st) : launch_cg<1>(cl, P, smem, st);
+}
+
+cudaError_t res_launch_cgstab(int sto, bool comp, const ResP &P, size_t smem, cudaStream_t st) {
+  if (sto == 3)
+    return comp ? launch(k_cgstab_res<3, true>, false, P, smem, st)
+                : launch(k_cgstab_res<3, false>, false, P, smem, st);
+  return comp ? launch(k_cgstab_res<1, true>, false, P, smem, st)
+              : launch(k_cgstab_res<1, false>, false, P, smem, st);
 }
 
 template <int STO, int COM>

@@ -66,6 +66,8 @@ struct ResP {
   int keep;                   // steps whose slots are loaded to stay in L2
   double eps;
   double *r, *ad;
+  // k_cgstab_res (r, ad: R and V published)
+  double *tv, *p0;
   // k_mixed_res
   int max_outer, max_inner;
   double outer_tol, inner_tol;
@@ -103,6 +105,7 @@ __host__ __device__ inline ResLayout res_layout(int own, int halo, int G, bool c
 // Launchers (bief_resident.cu); they return cudaGetLastError()'s value.
 cudaError_t res_launch_plan(bool fill, const PlanP &A, cudaStream_t st);
 cudaError_t res_launch_cg(int sto, bool cl, const ResP &P, size_t smem, cudaStream_t st);
+cudaError_t res_launch_cgstab(int sto, bool comp, const ResP &P, size_t smem, cudaStream_t st);
 // shift: 0 when the local indices are byte offsets, else 2.
 cudaError_t res_launch_mixed(int sto, bool cl, bool vs, int shift, const ResP &P, size_t smem,
                              cudaStream_t st);
