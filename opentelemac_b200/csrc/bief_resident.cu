@@ -1402,10 +1402,30 @@ __global__ void __launch_bounds__(MT, 1) k_mixed_res(const __grid_constant__ Res
       H.each(Q, hsrc, [&](int h, float rv) {
         win[Q.own + h] = start ? rv : add(rv, mul(beta, win[Q.own + h]));
       });
-      rows([&](int, int a, int i) {
-        const float rv = VS ? s_r[a] : P.ri[i];
-        win[a] = start ? rv : add(rv, mul(beta, win[a]));
-      });
+      if constexpr (VS) {
+        rows([&](int, int a, int) {
+          win[a] = start ? s_r[a] : add(s_r[a], mul(beta, win[a]));
+        });
+      } else {
+#pragma unroll 1
+        for (int v = 0; v < V; ++v) {
+          const int hi = N.hi(v);
+          int i = N.lo(v);
+          float *wa = win + (size_t)v * R * TP + t;
+#pragma unroll 1
+          for (; i + 3 * RES_T < hi; i += 4 * RES_T, wa += 4 * RES_T) {
+            float rv[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) rv[c] = P.ri[i + c * RES_T];
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              wa[c * RES_T] = start ? rv[c] : add(rv[c], mul(beta, wa[c * RES_T]));
+          }
+#pragma unroll 1
+          for (; i < hi; i += RES_T, wa += RES_T)
+            *wa = start ? P.ri[i] : add(P.ri[i], mul(beta, *wa));
+        }
+      }
       __syncthreads();
       start = false;
       sf[0] = sf[1] = 0.0f;

@@ -1,0 +1,167 @@
+"""The solvers that keep their search direction in shared memory, bit for bit
+against the oracle at the sizes where their forms change: one tree block up to
+8 (a cluster; 2,048 nodes per block), 9 to 24 (tagged partial sums), more (an
+arrival counter), more tree blocks than SMs (two per physical block), with
+uneven last blocks, unstructured node degrees (odd slice widths) and both
+storages.  Iterations are capped: every form runs a few dozen."""
+import numpy as np
+import pytest
+
+from opentelemac_b200 import bief, meshgen as mg
+
+pytestmark = pytest.mark.gpu
+
+
+def _grid(nx, ny, seed=3):
+    """nx x ny jittered grid, quads cut along random diagonals."""
+    rng = np.random.default_rng([seed, nx, ny])
+    i, j = np.meshgrid(np.arange(nx), np.arange(ny), indexing="xy")
+    x = ((i + rng.uniform(-0.2, 0.2, i.shape)) / nx).ravel()
+    y = ((j + rng.uniform(-0.2, 0.2, i.shape)) / nx).ravel()
+    a = (np.arange(ny - 1)[:, None] * nx + np.arange(nx - 1)).ravel()
+    b, c, d = a + 1, a + nx + 1, a + nx
+    cut = (rng.random(a.size) < 0.5)[:, None]
+    ik = np.empty((2 * a.size, 3), dtype=np.int32)
+    ik[0::2] = np.where(cut, np.stack([a, b, d], 1), np.stack([a, b, c], 1))
+    ik[1::2] = np.where(cut, np.stack([b, c, d], 1), np.stack([a, c, d], 1))
+    return x, y, ik
+
+
+# (nx, ny, tree blocks)
+SIZES = [(2, 2, 1), (5, 7, 1), (32, 64, 1), (33, 63, 2), (128, 128, 8), (129, 128, 9),
+         (224, 219, 24), (225, 221, 25)]
+
+
+def _problem(oracle_mod, x, y, ik, seed=1):
+    dm, xm = oracle_mod.wave_matrix(x, y, ik, mg.wave_coef(mg.depth_smooth(x, y, ik)))
+    xt = np.random.default_rng(seed).uniform(-1, 1, x.size)
+    b = oracle_mod.matvec("X=AY    ", ik, dm, "Q", xm, "S", xt)
+    return dm, xm, b
+
+
+def _stored(oracle_mod, ik, n, dm, xm, typext, storage, bps=0):
+    mesh = bief.Mesh(ik, n)
+    if bps:
+        mesh.set_blocks_per_sm(bps)
+    A = bief.Matrix(mesh, dm, xm, "Q", typext)
+    seg = None
+    if storage == "seg":
+        g1, g2, es, ori = mg.segments(ik, n)
+        mesh.set_segments(g1, g2)
+        A.to_segments()
+        seg = (g1, g2, oracle_mod.assex3(es, ori, typext, xm, g1.size))
+    return mesh, A, seg
+
+
+def _check_solve(oracle_mod, ik, n, dm, xm, typext, b, storage, slv, nitmax, x0, modass=1, bps=0):
+    mesh, A, seg = _stored(oracle_mod, ik, n, dm, xm, typext, storage, bps)
+    G, T = mesh.launch_info()
+    x = x0.copy()
+    cfg = bief.SlvCfg(slv=slv, nitmax=nitmax, precon=2, krylov=0, eps=1e-9, zero=0.0)
+    st, nit, relres = bief.solve(x, A, b.copy(), cfg, modass=modass)
+    mode = oracle_mod.DOT_BLOCKED if modass == 1 else oracle_mod.DOT_COMP_BLOCKED
+    kw = dict(slv=slv, eps=1e-9, nitmax=nitmax, x0=x0, dot_mode=mode, nblocks=G, nthreads=T)
+    with oracle_mod.threads():
+        if seg:
+            r = oracle_mod.solve_seg(seg[0], seg[1], dm, "Q", seg[2], typext, b, **kw)
+        else:
+            r = oracle_mod.solve(ik, dm, "Q", xm, typext, b, **kw)
+    assert (st, nit, relres) == (r["status"], r["nit"], r["relres"])
+    np.testing.assert_array_equal(x, r["x"])
+    # again on the same handle, the plan in place
+    x = x0.copy()
+    assert bief.solve(x, A, b.copy(), cfg, modass=modass)[1] == nit
+    np.testing.assert_array_equal(x, r["x"])
+    mesh.close()
+    return G
+
+
+def _check_mixed(oracle_mod, ik, n, dm, xm, b, storage, max_inner, bps=0):
+    mesh, A, seg = _stored(oracle_mod, ik, n, dm, xm, "S", storage, bps)
+    G, T = mesh.launch_info()
+    x = np.zeros(n)
+    st, outer, inner, relres = bief.solve_mixed(x, A, b, precon=2, inner_tol=0.1,
+                                                outer_tol=1e-10, max_inner=max_inner)
+    kw = dict(precon=2, inner_tol=0.1, outer_tol=1e-10, max_outer=1000, max_inner=max_inner,
+              nblocks=G, nthreads=T)
+    with oracle_mod.threads():
+        if seg:
+            r = oracle_mod.solve_mixed_seg(seg[0], seg[1], dm, "Q", seg[2], b, **kw)
+        else:
+            r = oracle_mod.solve_mixed(ik, dm, "Q", xm, b, **kw)
+    assert (st, outer, inner, relres) == (r["status"], r["outer"], r["inner"], r["relres"])
+    np.testing.assert_array_equal(x, r["x"])
+    # the binary32 product rebuilds its own slots after the solve's paired ones
+    import torch
+    xs = torch.tensor(b, device="cuda", dtype=torch.float32)
+    y1, y2 = torch.empty_like(xs), torch.empty_like(xs)
+    bief.matvec32(y1, A, xs)
+    bief.solve_mixed(np.zeros(n), A, b, precon=2, inner_tol=0.1, outer_tol=1e-10, max_inner=3)
+    bief.matvec32(y2, A, xs)
+    assert torch.equal(y1, y2)
+    mesh.close()
+
+
+@pytest.mark.parametrize("storage", ["ebe", "seg"])
+@pytest.mark.parametrize("nx,ny,blocks", SIZES)
+def test_forms_bitexact(oracle_mod, nx, ny, blocks, storage):
+    x, y, ik = _grid(nx, ny)
+    n = x.size
+    dm, xm, b = _problem(oracle_mod, x, y, ik)
+    x0 = np.random.default_rng(5).uniform(-0.1, 0.1, n)
+    assert _check_solve(oracle_mod, ik, n, dm, xm, "S", b, storage, 1, 40, x0) == blocks
+    _check_mixed(oracle_mod, ik, n, dm, xm, b, storage, 60)
+
+
+@pytest.mark.parametrize("modass", [1, 3])
+@pytest.mark.parametrize("typext,storage", [("S", "ebe"), ("Q", "ebe"), ("Q", "seg")])
+def test_cgstab_bitexact(oracle_mod, typext, storage, modass):
+    """CGSTAB's shared-memory form (9 tree blocks and more)."""
+    x, y, ik = _grid(150, 141)
+    n = x.size
+    dm, xm, b = _problem(oracle_mod, x, y, ik)
+    if typext == "Q":
+        rng = np.random.default_rng(2)
+        xm = np.concatenate([xm, xm * (1 + 0.05 * rng.uniform(-1, 1, xm.shape))])
+    assert _check_solve(oracle_mod, ik, n, dm, xm, typext, b, storage, 6, 25, np.zeros(n),
+                        modass) > 8
+
+
+@pytest.mark.parametrize("npts", [3000, 24000, 60000])
+def test_random_numbering(oracle_mod, npts):
+    """Points numbered at random: the halo is most of the mesh."""
+    x, y, ik = mg.delaunay_mesh(npts)
+    n = x.size
+    dm, xm, b = _problem(oracle_mod, x, y, ik)
+    _check_solve(oracle_mod, ik, n, dm, xm, "S", b, "ebe", 1, 25, np.zeros(n))
+    _check_mixed(oracle_mod, ik, n, dm, xm, b, "ebe", 30)
+
+
+def test_two_tree_blocks_per_block(oracle_mod):
+    """More tree blocks than SMs (two blocks per SM asked for on a mesh of an
+    odd number of them): two tree blocks per physical block, the last alone."""
+    x, y, ik = _grid(601, 599)
+    n = x.size
+    dm, xm, b = _problem(oracle_mod, x, y, ik)
+    G = _check_solve(oracle_mod, ik, n, dm, xm, "S", b, "ebe", 1, 8, np.zeros(n), bps=2)
+    assert G > 148
+    _check_mixed(oracle_mod, ik, n, dm, xm, b, "ebe", 12, bps=2)
+
+
+def test_zero_rhs_and_breakdown(oracle_mod):
+    """B = 0 and an indefinite matrix, in each form."""
+    for nx, ny in ((20, 21), (150, 141), (240, 230)):
+        x, y, ik = _grid(nx, ny)
+        n = x.size
+        dm, xm, b = _problem(oracle_mod, x, y, ik)
+        mesh = bief.Mesh(ik, n)
+        A = bief.Matrix(mesh, dm, xm, "Q", "S")
+        cfg = bief.SlvCfg(slv=1, nitmax=50, precon=2, krylov=0, eps=1e-8, zero=0.0)
+        u = np.ones(n)
+        assert bief.solve(u, A, np.zeros(n), cfg)[:2] == (0, 0) and not u.any()
+        u = np.ones(n)
+        assert bief.solve_mixed(u, A, np.zeros(n))[0] == 0 and not u.any()
+        A.set(dm, 3.0 * xm, "Q", "S")
+        with pytest.raises(bief.BiefError):
+            bief.solve(np.zeros(n), A, b.copy(), cfg)
+        mesh.close()
