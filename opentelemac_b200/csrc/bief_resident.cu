@@ -292,7 +292,8 @@ __device__ __forceinline__ T tag_value(unsigned long long x, unsigned long long 
 
 // How the blocks of a solve talk to each other.
 //   COM_CL   cluster: every warp's total goes straight to every block's shared
-//            memory as tagged words, halo values are read from there;
+//            memory, each with an arrival on that block's mbarrier; halo values
+//            are read from the owner's shared memory;
 //   COM_TAG  grid: block totals as tagged words that all blocks poll;
 //   COM_CNT  grid: block totals and an arrival counter.
 // Measured per reduction in a loop of nothing else at 1024 threads (us):
@@ -329,18 +330,20 @@ struct Comm {
     ++nbar;
     if constexpr (CL) {
       const T u = warp_tree(v[0]);
-      if (PUB) {
-        __syncwarp();
-        fence_cluster();
-      }
+      __syncwarp();  // the warp's writes before its lanes' releases
       if (lane < NP) {
         const int vw = (p % S) * ((int)blockDim.x >> 5) + w;
         const int slot = (p / S) * 32 + vw;
         const unsigned a =
-            mapa(smem_addr(box + 2 * ((size_t)(nbar & 1) * 32 * G + slot)), (unsigned)lane);
-        tag_words(u, nbar, x, y);
-        asm volatile("st.relaxed.cluster.shared::cluster.v2.b64 [%0], {%1, %2};" ::"r"(a), "l"(x),
-                     "l"(y)
+            mapa(smem_addr(box + (size_t)(nbar & 1) * 32 * G + slot), (unsigned)lane);
+        if constexpr (sizeof(T) == 8)
+          asm volatile("st.relaxed.cluster.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"((double)u)
+                       : "memory");
+        else
+          asm volatile("st.relaxed.cluster.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"((float)u)
+                       : "memory");
+        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(
+                         mapa(smem_addr(&sh->mbar[nbar & 1]), (unsigned)lane))
                      : "memory");
       }
     } else {
@@ -386,35 +389,44 @@ struct Comm {
       ns = CL ? G : (G + 31) >> 5;
       if (w < ns) {
         T u = T(0);
-        if (CL || t < G) {
-          const unsigned long long *m =
-              box + 2 * ((size_t)(nbar & 1) * (CL ? 32 : 1) * G + t);
+        if constexpr (CL) {
+          const unsigned bar = smem_addr(&sh->mbar[nbar & 1]), par = ((nbar - 1) >> 1) & 1;
+          unsigned ok = 0;
+          unsigned long long t0 = 0;
+#pragma unroll 1
+          for (unsigned n = 1;; ++n) {  // each try waits in hardware, for a bounded time
+            asm volatile(
+                "{\n.reg .pred p;\n"
+                "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                "selp.u32 %0, 1, 0, p;\n}"
+                : "=r"(ok)
+                : "r"(bar), "r"(par)
+                : "memory");
+            if (ok) break;
+            if ((n & 0xf) == 0) {
+              if (!t0) t0 = global_ns();
+              else if ((long long)(global_ns() - t0) > timeout_ns) { bad = 1; break; }
+            }
+          }
+          u = *reinterpret_cast<const volatile T *>(box + (size_t)(nbar & 1) * 32 * G + t);
+        } else if (t < G) {
+          const unsigned long long *m = box + 2 * ((size_t)(nbar & 1) * G + t);
           unsigned long long x, y, t0 = 0;
 #pragma unroll 1
           for (unsigned n = 1;; ++n) {
-            if constexpr (CL)
-              asm volatile("ld.relaxed.cluster.shared::cta.v2.b64 {%0, %1}, [%2];"
-                           : "=l"(x), "=l"(y)
-                           : "r"(smem_addr(m))
-                           : "memory");
-            else
-              asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];"
-                           : "=l"(x), "=l"(y)
-                           : "l"(m)
-                           : "memory");
+            asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];"
+                         : "=l"(x), "=l"(y)
+                         : "l"(m)
+                         : "memory");
             if ((unsigned)x == nbar && (unsigned)y == nbar) break;
             if ((n & 0xff) == 0) {
               if (!t0) t0 = global_ns();
               else if ((long long)(global_ns() - t0) > timeout_ns) { bad = 1; break; }
             }
           }
-          u = tag_value<T>(x, y);
-          if (!CL) u = add(T(0), u);
+          u = add(T(0), tag_value<T>(x, y));
         }
-        if (PUB) {
-          if (CL) fence_cluster();
-          else fence_gpu();
-        }
+        if (PUB && !CL) fence_gpu();
         __syncwarp();
         u = warp_tree(u);
         if (lane == 0) reinterpret_cast<T *>(sh->us[nbar & 1])[w] = u;
@@ -833,7 +845,14 @@ __device__ __forceinline__ void comm_init(Comm<COM> &M, const ResP &P, int V, un
   M.nbar = 0;
   if (COM == COM_CL)
 #pragma unroll 1
-    for (int i = threadIdx.x; i < 2 * 32 * M.G * 2; i += blockDim.x) M.box[i] = 0;
+    if (threadIdx.x == 0) {
+      // one arrival per warp of the cluster and reduction
+      for (int q = 0; q < 2; ++q)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&M.sh->mbar[q])),
+                     "r"(32 * M.G)
+                     : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -876,7 +895,7 @@ __global__ void __launch_bounds__(MT, 1) k_cg_res(const __grid_constant__ ResP P
   Comm<COM> M;
   comm_init(M, P, V, res_sm + L.red, res_sm + L.box);
   res_setup<C, I, 1>(Q, p, P.S.meta, 0, P.S.rec_off, gc, gi, P.cache, s_off, s_deg, s_c, s_i);
-  if constexpr (CL) cluster_sync();  // every block of the cluster has cleared its box
+  if constexpr (CL) cluster_sync();  // every block's mbarriers are set up
   const bool vs = CL || P.nvec >= 2;
   const unsigned long long pol_keep = l2_policy(false), pol_stream = l2_policy(true);
   Ranges N;

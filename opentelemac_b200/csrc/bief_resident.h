@@ -39,6 +39,7 @@ struct PlanP {
 };
 
 struct RedShared {
+  unsigned long long mbar[2];
   double ws[2][32];
   double cold[3];   // scalars of the mixed solve
   double us[2][16];  // alternate: a warp may still read the previous reduction's
@@ -93,7 +94,7 @@ __host__ __device__ inline ResLayout res_layout(int own, int halo, int G, bool c
   L.win = take((size_t)elt * (size_t)(own + halo));
   L.vec = take((size_t)elt * own * nvec);
   L.red = take(sizeof(RedShared));
-  L.box = take(cl ? (size_t)2 * 32 * G * 16 : 0);
+  L.box = take(cl ? (size_t)2 * 32 * G * 8 : 0);
   L.off = take(sizeof(int2) * (size_t)(own / 32));
   L.deg = take((size_t)own);
   L.ccoef = take((size_t)cb * cache);
