@@ -513,7 +513,7 @@ def config2_measure(P2, ws, flush_l2, hbm, steps=2, warmup=1):
         out[key] = {"ms": ms, "kernel_ms": kern, "inner": inner, "refinements": outer,
                     "relres": relres, "speedup_vs_fp64": f64_ms / ms,
                     "vs_fp64": nrm(x - x64) / nrm(x64), "vs_tight_fp64": nrm(x - x13) / nrm(x13),
-                    "kernel": "k_mixed", "gbs": mb / (kern * 1e-3) / 1e9,
+                    "kernel": "k_mixed_res", "gbs": mb / (kern * 1e-3) / 1e9,
                     "frac": mb / (kern * 1e-3) / 1e9 / hbm, "bytes_per_launch": mb}
     del x, x64, x13
     return out
@@ -1002,7 +1002,7 @@ def main():
         pass
     mixed_bytes = inner * by["it32"] + (outer + 1) * by["upd"]
     achieved = mixed_bytes / (kern_ms * 1e-3) / 1e9
-    mixed_traffic = traffic.get("k_mixed_bytes_per_launch")
+    mixed_traffic = traffic.get("k_mixed_res_bytes_per_launch")
     dram_gbs = mixed_traffic / (kern_ms * 1e-3) / 1e9 if mixed_traffic else None
     # the binary32 operator and vectors of the 1M-node solve (~96 MB) fit in
     # the 126 MB L2: whether the launch's working set stays in L2
@@ -1048,11 +1048,11 @@ def main():
             "fp64_modass3": {"ms": sum(c64_ms) / len(c64_ms), "iterations": c64_res[1],
                              "vs_fp64": c64_vs_f64,
                              "note": "GRACJG with compensated dot products (MODASS=3)"},
-            "fp64_cg": {"kernel": "k_cg64", "gbs": f64_bytes / (f64_kern_ms * 1e-3) / 1e9,
+            "fp64_cg": {"kernel": "k_cg_res", "gbs": f64_bytes / (f64_kern_ms * 1e-3) / 1e9,
                         "frac": f64_bytes / (f64_kern_ms * 1e-3) / 1e9 / hbm,
                         "bytes_per_iteration": by["it64"], "bytes_per_launch": f64_bytes,
-                        "traffic": traffic.get("k_cg64_bytes_per_launch")},
-            "roofline": {"bound": "hbm", "kernel": "k_mixed", "achieved": achieved,
+                        "traffic": traffic.get("k_cg_res_bytes_per_launch")},
+            "roofline": {"bound": "hbm", "kernel": "k_mixed_res", "achieved": achieved,
                          "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                          "peak_source": f"{peak_src} (MEASURED_PEAKS.json hbm_gbs)",
                          "bytes_per_launch": mixed_bytes,

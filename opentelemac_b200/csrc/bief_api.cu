@@ -425,8 +425,8 @@ int res_ensure(bief_handle *h, cudaStream_t st) {
     const long long hi = b + 1 >= Q.G ? Q.n : (((long long)(b + 1) * Q.n / Q.G) & ~31LL);
     Q.R = std::max(Q.R, (int)((hi - lo + RES_T - 1) / RES_T));
   }
-  // Up to 8 tree blocks (16,384 nodes): one cluster, each tree block's warps
-  // shared out over as many of its blocks as there are.
+  // Up to RES_MAXCL tree blocks (24,576 nodes): one cluster, each tree block's
+  // warps shared out over as many of its blocks as there are.
   h->res_cl = false;
   if (Q.G <= RES_MAXCL && Q.R <= 2) {
     int S = 1;

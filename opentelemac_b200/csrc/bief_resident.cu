@@ -18,8 +18,8 @@
 //   CL = false  one physical block per SM holding V virtual blocks (V = 2
 //               when the tree has more blocks than SMs), grid barriers
 //               through global memory;
-//   CL = true   meshes of up to 16 virtual blocks (32,768 nodes): one cluster
-//               of G*S blocks, each holding 1/S of a virtual block's warps;
+//   CL = true   meshes of up to 12 virtual blocks (24,576 nodes): one cluster
+//               of G*S <= 12 blocks, each holding 1/S of a virtual block's warps;
 //               partial sums and halo values through distributed shared
 //               memory.
 #include <type_traits>
@@ -88,17 +88,30 @@ __global__ void __launch_bounds__(1024, 1) k_res_plan(PlanP A) {
     s_run = 0;
   }
   __syncthreads();
+  // the block's own node ranges (res_node and res_local for this block,
+  // without their 64-bit divisions)
+  const int b0 = Q.V > 1 ? p * Q.V : p / Q.S, s0 = Q.V > 1 ? 0 : (p % Q.S) * Q.TP;
+  const int L0 = (int)blk_lo(b0, Q.n, Q.G), L1 = (int)blk_lo(b0 + 1, Q.n, Q.G);
+  const int L2 = Q.V > 1 && b0 + 1 < Q.G ? (int)blk_lo(b0 + 2, Q.n, Q.G) : L1;
   auto each_row = [&](auto f) {
 #pragma unroll 1
     for (int a = t; a < Q.own; a += T) {
-      const int i = res_node(Q, p, a / Q.TP, a % Q.TP);
-      if (i >= 0) f(i);
+      const int kk = a / Q.TP, v = kk / Q.R;
+      const int i = (v ? L1 : L0) + s0 + a % Q.TP + RES_T * (kk - v * Q.R);
+      if (i < (v ? L2 : L1)) f(i);
     }
   };
   auto outside = [&](int j, int &loc) {
-    int pp;
-    res_local(Q, j, pp, loc);
-    return pp != p;
+    int v = 0, off = j - L0;
+    if (j >= L1) {
+      v = 1;
+      off = j - L1;
+      if (j >= L2) return true;
+    }
+    if (off < 0) return true;
+    const int k = off / RES_T, vt = off % RES_T - s0;
+    loc = (v * Q.R + k) * Q.TP + vt;
+    return vt < 0 || vt >= Q.TP;
   };
   int mn = 0x7fffffff, mx = -1;
   each_row([&](int i) {
@@ -863,6 +876,9 @@ __device__ __forceinline__ void comm_init(Comm<COM> &M, const ResP &P, int V, un
 // code, told apart by `phase`, and loops stay rolled: unrolled or repeated,
 // the loop outgrew the instruction caches, and with most of the SM's memory
 // taken as shared memory every register spill is an L2 access.
+// Bound: the reductions and dependent binary64 chains on small meshes (1,681
+// nodes 10.7 -> 3.5 us per iteration against k_cg64), window conflicts and two
+// grid reductions at 150k (18 -> 12), the records' bytes at 1.0M (34 -> 26.8).
 // ---------------------------------------------------------------------------
 template <int STO, int COM, int MT>
 __global__ void __launch_bounds__(MT, 1) k_cg_res(const __grid_constant__ ResP P) {
@@ -1092,6 +1108,8 @@ __global__ void __launch_bounds__(MT, 1) k_cg_res(const __grid_constant__ ResP P
 // nodes and of its halo are in shared memory: the halo's copies follow by
 // their owners' operations from one value per product (V, then T), where
 // k_cgstab gathered three vectors per neighbour for A Q and two for A S.
+// Bound: three grid reductions and two products (100k nodes 37.4 -> 27.0 us
+// per iteration, 300k 29.8 -> 25.5).
 // ---------------------------------------------------------------------------
 template <int STO, bool COMP>
 __global__ void __launch_bounds__(RES_T, 1) k_cgstab_res(const __grid_constant__ ResP P) {
@@ -1299,6 +1317,9 @@ __device__ __noinline__ ResidualSums mixed_residual(const ResP &P, float *s_r) {
 // Mixed precision, statement for statement k_mixed.  VS: r, q and z of the
 // own rows and their row sums in shared memory (always in the cluster form);
 // else in global memory.  SH = 0: local indices as byte offsets.
+// Bound: reductions (5.2 of 12.7 us per iteration at 1.0M nodes; k_mixed 16.4)
+// and the latency of the slots that are not in shared memory; at 4.0M nodes
+// HBM, 184 MB per iteration (78 -> 53 us).
 // ---------------------------------------------------------------------------
 template <int STO, int COM, bool VS, int SH, int MT>
 __global__ void __launch_bounds__(MT, 1) k_mixed_res(const __grid_constant__ ResP P) {

@@ -7,9 +7,12 @@
 namespace bief {
 
 constexpr int RES_T = 1024;      // threads of a virtual block (the tree's)
-// Blocks of a cluster.  A reduction in a cluster of 16 (not portable) takes
-// 4,500-5,000 cycles against 1,900-2,200 in one of 8.
-constexpr int RES_MAXCL = 8;
+// Blocks of a cluster.  Measured with at most 8 against at most 16 (us per
+// iteration, binary64 / mixed): 1 tree block as 8 or 16 blocks 3.51 / 3.21
+// against 3.89 / 3.61; 6 tree blocks as 6 or 12, binary64, 7.31 against 5.39;
+// 11 tree blocks in the grid form or as 11, 9.05 / 7.47 against 8.67 / 6.73;
+// 15 tree blocks likewise 8.89 / 6.90 against 10.0 / 8.34.
+constexpr int RES_MAXCL = 12;
 constexpr int RES_TAG = 24;  // grid blocks up to which partial sums are tagged words
 
 // Partition of the nodes over physical blocks, and the local index lists.
