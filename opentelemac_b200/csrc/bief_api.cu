@@ -447,6 +447,10 @@ int res_ensure(bief_handle *h, cudaStream_t st) {
   Q.halo_off = h->d_res_off;
   PlanP A = {};
   A.Q = Q;
+  const bool sg = h->has_segments != 0;
+  A.nb_meta = sg ? h->d_sg_meta : h->d_meta;
+  A.nb_off = sg ? h->d_sg_off : h->d_seg_off;
+  A.nb_col = sg ? h->d_sg_col : h->d_seg_col;
   A.meta = h->d_meta;
   A.seg_off = h->d_seg_off;
   A.seg_col = h->d_seg_col;
@@ -465,7 +469,6 @@ int res_ensure(bief_handle *h, cudaStream_t st) {
     total += c;
   }
   if (Q.own + most > 0xffff) return BIEF_OK;
-  const bool sg = h->has_segments != 0;
   if (!h->res_cl && (stt = dalloc(&h->d_res_box, res_box_words(Q.G)))) return stt;
   if ((stt = dalloc(&h->d_res_halo, (size_t)total)) || (stt = dalloc(&h->d_res_loc, (size_t)total)) ||
       (stt = dalloc(&h->d_seg_li, (size_t)h->nseg)) || (stt = dalloc(&h->d_rec_li, (size_t)h->nrec + 32)) ||

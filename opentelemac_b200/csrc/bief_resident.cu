@@ -115,11 +115,11 @@ __global__ void __launch_bounds__(1024, 1) k_res_plan(PlanP A) {
   };
   int mn = 0x7fffffff, mx = -1;
   each_row([&](int i) {
-    const int nn = A.meta[i] >> 16, b = A.seg_off[i >> 5] + (i & 31);
+    const int nn = A.nb_meta[i] >> 16, b = A.nb_off[i >> 5] + (i & 31);
 #pragma unroll 1
     for (int m = 0; m < nn; ++m) {
       int loc;
-      const int j = A.seg_col[b + 32 * m];
+      const int j = A.nb_col[b + 32 * m];
       if (outside(j, loc)) {
         mn = min(mn, j);
         mx = max(mx, j);
@@ -139,11 +139,11 @@ __global__ void __launch_bounds__(1024, 1) k_res_plan(PlanP A) {
     for (int q = t; q < PLAN_W; q += T) bits[q] = 0;
     __syncthreads();
     each_row([&](int i) {
-      const int nn = A.meta[i] >> 16, b = A.seg_off[i >> 5] + (i & 31);
+      const int nn = A.nb_meta[i] >> 16, b = A.nb_off[i >> 5] + (i & 31);
 #pragma unroll 1
       for (int m = 0; m < nn; ++m) {
         int loc;
-        const int j = A.seg_col[b + 32 * m];
+        const int j = A.nb_col[b + 32 * m];
         if (inside(j) && outside(j, loc)) atomicOr(&bits[(j - lo) >> 5], 1u << (j & 31));
       }
     });

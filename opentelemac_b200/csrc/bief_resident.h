@@ -29,7 +29,10 @@ constexpr int PLAN_W = 20480;
 
 struct PlanP {
   ResPart Q;
-  const int *meta, *seg_off, *seg_col;   // distinct neighbours (halo)
+  // neighbours that make the halo: the segments' when there are segments (each
+  // element face is one, and a segment need not be a face), else the mesh's
+  const int *nb_meta, *nb_off, *nb_col;
+  const int *meta, *seg_off, *seg_col;   // binary32 slots: distinct neighbours
   const int *rec_off;                    // records: meta's low half entries
   const int2 *rec_idx;
   const int *sg_meta, *sg_off, *sg_col;  // segment slots, when sg_li

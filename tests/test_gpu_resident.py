@@ -165,3 +165,50 @@ def test_zero_rhs_and_breakdown(oracle_mod):
         with pytest.raises(bief.BiefError):
             bief.solve(np.zeros(n), A, b.copy(), cfg)
         mesh.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(60, 61), (171, 161), (251, 241)])
+def test_segments_that_are_no_face(oracle_mod, nx, ny):
+    """A segment need not be an element's face: its far node belongs to the
+    halo all the same (each form; GRACJG, CGSTAB and the mixed solve)."""
+    x, y, ik = _grid(nx, ny)
+    n = x.size
+    dm, xm, _ = _problem(oracle_mod, x, y, ik)
+    g1, g2, es, ori = mg.segments(ik, n)
+    xa = oracle_mod.assex3(es, ori, "S", xm, g1.size)
+    face = set(zip(np.minimum(g1, g2).tolist(), np.maximum(g1, g2).tolist()))
+    rng = np.random.default_rng(nx)
+    far = [(0, n - 1), (n // 2, 1), (n - 2, n // 3)]  # and at random over the mesh
+    for a, b in rng.integers(0, n, (40, 2)).tolist():
+        k = (min(a, b), max(a, b))
+        if a != b and k not in face and k not in {(min(p), max(p)) for p in far}:
+            far.append((a, b))
+    g1 = np.concatenate([g1, [p[0] for p in far]])
+    g2 = np.concatenate([g2, [p[1] for p in far]])
+    xa = np.concatenate([xa.ravel(), -0.3 * dm.mean() * rng.uniform(0.5, 1.0, len(far))])
+    dm = dm.copy()
+    for a, b in far:  # diagonally as dominant as before
+        dm[a] += 0.4 * dm.mean()
+        dm[b] += 0.4 * dm.mean()
+    b = rng.uniform(-1, 1, n) * dm
+    mesh = bief.Mesh(ik, n)
+    mesh.set_segments(g1, g2)
+    A = bief.Matrix(mesh).set_seg(dm, xa)
+    G, T = mesh.launch_info()
+    for slv in (1, 6):
+        u = np.zeros(n)
+        cfg = bief.SlvCfg(slv=slv, nitmax=25, precon=2, krylov=0, eps=1e-9, zero=0.0)
+        st, nit, relres = bief.solve(u, A, b.copy(), cfg)
+        with oracle_mod.threads():
+            r = oracle_mod.solve_seg(g1, g2, dm, "Q", xa, "S", b, slv=slv, eps=1e-9, nitmax=25,
+                                     dot_mode=oracle_mod.DOT_BLOCKED, nblocks=G, nthreads=T)
+        assert (st, nit, relres) == (r["status"], r["nit"], r["relres"])
+        np.testing.assert_array_equal(u, r["x"])
+    u = np.zeros(n)
+    got = bief.solve_mixed(u, A, b, inner_tol=0.1, outer_tol=1e-10, max_inner=40)
+    with oracle_mod.threads():
+        r = oracle_mod.solve_mixed_seg(g1, g2, dm, "Q", xa, b, inner_tol=0.1, outer_tol=1e-10,
+                                       max_inner=40, nblocks=G, nthreads=T)
+    assert got == (r["status"], r["outer"], r["inner"], r["relres"])
+    np.testing.assert_array_equal(u, r["x"])
+    mesh.close()
