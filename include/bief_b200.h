@@ -267,6 +267,12 @@ int bief_diri01_dev(bief_handle *h, int nptfr, const int *nbor,
  * wait with a 2 s limit. */
 int bief_selftest_timeout(int device, long long timeout_ns);
 
+/* The limit of dynamic shared memory now set for the GRACJG kernel of meshes
+ * of a few thousand nodes (no reference counterpart).  It belongs to the
+ * kernel, not to a handle: no solve may leave it below what another handle's
+ * solve, perhaps from another thread, needs. */
+int bief_selftest_smem(int device, int *bytes);
+
 /* Shape of the device dot-product tree: number of blocks and threads per
  * block of the persistent solver kernel. */
 int bief_launch_info(bief_handle *h, int *nblocks, int *nthreads);

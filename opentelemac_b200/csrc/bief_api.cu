@@ -656,6 +656,7 @@ ResP res_params(const bief_handle *h, const CP &C, int td) {
   P.box = h->d_res_box;
   P.timeout_ns = C.timeout_ns;
   P.halo_max = h->res_halo_max;
+  P.smem_limit = h->smem_max;
   return P;
 }
 
@@ -703,6 +704,7 @@ int res_cgstab(bief_handle *h, const StabP &C, int td, bool comp, cudaStream_t s
   if (layout(0) + fixed > (size_t)h->smem_max) return BIEF_OK;
   ResP P = res_params(h, C, td);
   P.cache = res_cache_slots(h, layout(0) + fixed, cb + ib);
+  P.smem_limit = h->smem_max - (int)fixed;
   P.nitmax = C.nitmax;
   P.eps = C.eps;
   P.keep = res_keep(h, C.S.cs_rec != 0, cb + ib);
@@ -1881,6 +1883,13 @@ int bief_selftest_timeout(int device, long long timeout_ns) {
   cudaFree(ctl);
   if (e != cudaSuccess) return cuda_fail(e, "selftest", __LINE__);
   return host.status == ST_TIMEOUT ? BIEF_ERR_DEVICE_TIMEOUT : BIEF_ERR_CUDA;
+}
+
+int bief_selftest_smem(int device, int *bytes) {
+  if (!bytes) return BIEF_ERR_ARGS;
+  DevGuard g(device);
+  CK(res_smem_limit(bytes));
+  return BIEF_OK;
 }
 
 int bief_launch_info(bief_handle *h, int *nblocks, int *nthreads) {

@@ -1613,9 +1613,15 @@ __global__ void __launch_bounds__(MT, 1) k_mixed_res(const __grid_constant__ Res
 // ---------------------------------------------------------------------------
 namespace {
 
+// The kernel's limit of dynamic shared memory is state of the context, shared
+// by every thread that launches the kernel: it is set to P.smem_limit, the
+// same for every mesh, and never to what one launch needs, which another
+// thread's launch might find too low (measured with three threads and two
+// sizes in a loop: 72 of 20,000 launches refused).
 template <class K>
 cudaError_t launch(K k, bool cl, const ResP &P, size_t smem, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e =
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, P.smem_limit);
   if (e != cudaSuccess) return e;
   if (cl && (e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) !=
                 cudaSuccess)
@@ -1703,6 +1709,13 @@ cudaError_t res_launch_mixed(int sto, bool cl, bool vs, int shift, const ResP &P
                              cudaStream_t st) {
   return sto == 3 ? launch_mixed<3>(cl, vs, shift, P, smem, st)
                   : launch_mixed<1>(cl, vs, shift, P, smem, st);
+}
+
+cudaError_t res_smem_limit(int *bytes) {
+  cudaFuncAttributes a;
+  const cudaError_t e = cudaFuncGetAttributes(&a, k_cg_res<1, COM_CL, RES_T / 2>);
+  *bytes = e == cudaSuccess ? a.maxDynamicSharedSizeBytes : 0;
+  return e;
 }
 
 bool res_cluster_fits(int np, int tp, size_t smem) {

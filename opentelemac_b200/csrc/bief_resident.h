@@ -67,6 +67,7 @@ struct ResP {
   long long timeout_ns;
   int cache;                  // operator slots (multiple of 32) kept in shared memory
   int halo_max;
+  int smem_limit;             // most dynamic shared memory a launch of the kernel may have
   int nvec;                   // own-row vectors in shared memory
   // k_cg_res
   int nitmax;
@@ -119,5 +120,9 @@ cudaError_t res_launch_mixed(int sto, bool cl, bool vs, int shift, const ResP &P
 // Whether a cluster of np blocks of tp threads with that much shared memory
 // can be resident (one probe for all cluster kernels).
 bool res_cluster_fits(int np, int tp, size_t smem);
+
+// The limit of dynamic shared memory that the cluster form's GRACJG (blocks
+// of at most 512 threads) has now.
+cudaError_t res_smem_limit(int *bytes);
 
 }  // namespace bief

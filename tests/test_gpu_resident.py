@@ -4,10 +4,12 @@ against the oracle at the sizes where their forms change: one tree block up to
 (an arrival counter), more tree blocks than SMs (two per physical block), with
 uneven last blocks, unstructured node degrees (odd slice widths) and both
 storages.  Iterations are capped: every form runs a few dozen."""
+import ctypes
+
 import numpy as np
 import pytest
 
-from opentelemac_b200 import bief, meshgen as mg
+from opentelemac_b200 import _native, bief, meshgen as mg
 
 pytestmark = pytest.mark.gpu
 
@@ -212,3 +214,53 @@ def test_segments_that_are_no_face(oracle_mod, nx, ny):
     assert got == (r["status"], r["outer"], r["inner"], r["relres"])
     np.testing.assert_array_equal(u, r["x"])
     mesh.close()
+
+
+def test_threads_with_their_own_handles():
+    """Two host threads, each with a mesh and a stream of its own: the launch
+    of one must not depend on the shared memory that the other's mesh asks
+    for (both meshes run the same kernel)."""
+    import threading
+    import torch
+    todo = []
+    for nx in (41, 90):
+        x, y, ik = _grid(nx, nx)
+        n = x.size
+        mesh = bief.Mesh(ik, n)
+        A = bief.Matrix(mesh, np.full(n, 8.0), np.full((3, ik.shape[0]), -0.5), "Q", "S")
+        b = torch.rand(n, device="cuda", dtype=torch.float64)
+        u = torch.empty_like(b)
+        todo.append((mesh, A, b, u, torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    errors = []
+    start = threading.Barrier(len(todo))
+
+    def work(mesh, A, b, u, stream):
+        cfg = bief.SlvCfg(slv=1, nitmax=2, precon=2, krylov=0, eps=1e-12, zero=0.0)
+        try:
+            with torch.cuda.stream(stream):
+                start.wait()
+                ref = None
+                for _ in range(1000):
+                    u.zero_()
+                    bief.solve(u, A, b, cfg)
+                    if ref is None:
+                        ref = u.clone()
+                assert torch.equal(u, ref)
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=a) for a in todo]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    # whichever solved last, the kernel's limit is the device's
+    limit = ctypes.c_int()
+    bief.solve(todo[0][3], todo[0][1], todo[0][2],
+               bief.SlvCfg(slv=1, nitmax=2, precon=2, krylov=0, eps=1e-12, zero=0.0))
+    assert _native.lib().bief_selftest_smem(0, ctypes.byref(limit)) == 0
+    assert limit.value == torch.cuda.get_device_properties(0).shared_memory_per_block_optin
+    for a in todo:
+        a[0].close()
