@@ -410,6 +410,23 @@ static int res_clear(bief_handle *h, cudaStream_t s) {
   return BIEF_OK;
 }
 
+// No plan: frees what there is of one, and the other kernels solve from now on.
+static int res_none(bief_handle *h) {
+  res_drop(h);
+  h->res_state = -1;
+  return BIEF_OK;
+}
+
+// Memory for the plan; false when there is none left, which is no error as
+// the kernels that need no plan can solve.
+template <typename T>
+static bool res_alloc(T **p, size_t n) {
+  if (cudaMalloc((void **)p, sizeof(T) * std::max<size_t>(n, 1)) == cudaSuccess) return true;
+  *p = nullptr;
+  cudaGetLastError();
+  return false;
+}
+
 int res_ensure(bief_handle *h, cudaStream_t st) {
   if (h->res_state) return BIEF_OK;
   h->res_state = -1;
@@ -442,8 +459,7 @@ int res_ensure(bief_handle *h, cudaStream_t st) {
   Q.NP = Q.V > 1 ? (Q.G + Q.V - 1) / Q.V : Q.G * Q.S;
   Q.own = Q.V * Q.R * Q.TP;
   if (Q.own > 0xffff) return BIEF_OK;
-  int stt;
-  if ((stt = dalloc(&h->d_res_off, (size_t)Q.NP + 1))) return stt;
+  if (!res_alloc(&h->d_res_off, (size_t)Q.NP + 1)) return res_none(h);
   Q.halo_off = h->d_res_off;
   PlanP A = {};
   A.Q = Q;
@@ -468,13 +484,14 @@ int res_ensure(bief_handle *h, cudaStream_t st) {
     cnt[p] = total;
     total += c;
   }
-  if (Q.own + most > 0xffff) return BIEF_OK;
-  if (!h->res_cl && (stt = dalloc(&h->d_res_box, res_box_words(Q.G)))) return stt;
-  if ((stt = dalloc(&h->d_res_halo, (size_t)total)) || (stt = dalloc(&h->d_res_loc, (size_t)total)) ||
-      (stt = dalloc(&h->d_seg_li, (size_t)h->nseg)) || (stt = dalloc(&h->d_rec_li, (size_t)h->nrec + 32)) ||
-      (sg && ((stt = dalloc(&h->d_sg_li, (size_t)h->nsg_slots + 32)) ||
-              (stt = dalloc(&h->d_sg_li2, (size_t)h->nsg_slots)))))
-    return stt;
+  if (Q.own + most > 0xffff) return res_none(h);
+  if ((!h->res_cl && !res_alloc(&h->d_res_box, res_box_words(Q.G))) ||
+      !res_alloc(&h->d_res_halo, (size_t)total) || !res_alloc(&h->d_res_loc, (size_t)total) ||
+      !res_alloc(&h->d_seg_li, (size_t)h->nseg) ||
+      !res_alloc(&h->d_rec_li, (size_t)h->nrec + 32) ||
+      (sg && (!res_alloc(&h->d_sg_li, (size_t)h->nsg_slots + 32) ||
+              !res_alloc(&h->d_sg_li2, (size_t)h->nsg_slots))))
+    return res_none(h);
   CK(cudaMemcpyAsync(h->d_res_off, cnt.data(), sizeof(int) * (Q.NP + 1), cudaMemcpyHostToDevice,
                      st));
   CK(cudaMemsetAsync(h->d_seg_li, 0, sizeof(short) * h->nseg, st));

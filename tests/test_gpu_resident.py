@@ -264,3 +264,42 @@ def test_threads_with_their_own_handles():
     assert limit.value == torch.cuda.get_device_properties(0).shared_memory_per_block_optin
     for a in todo:
         a[0].close()
+
+
+def test_no_memory_for_the_plan():
+    """A device with no memory left for a solver's plan: the kernels that need
+    none solve instead, with the same bits."""
+    import torch
+    nx, ny = 2001, 1001
+    k = np.arange(nx * ny).reshape(ny, nx)
+    a, b, c, d = (v.ravel() for v in (k[:-1, :-1], k[:-1, 1:], k[1:, 1:], k[1:, :-1]))
+    ik = np.concatenate([np.stack([a, b, c], 1), np.stack([a, c, d], 1)]).astype(np.int32)
+    n = nx * ny
+    rhs = torch.rand(n, device="cuda", dtype=torch.float64)
+
+    def handle():
+        mesh = bief.Mesh(ik, n)
+        return bief.Matrix(mesh, np.full(n, 8.0), np.full((3, ik.shape[0]), -0.5), "Q", "S")
+
+    def cg(A, u):
+        cfg = bief.SlvCfg(slv=1, nitmax=10, precon=2, krylov=0, eps=1e-13, zero=0.0)
+        return bief.solve(u, A, rhs, cfg)
+
+    def mixed(A, u):
+        return bief.solve_mixed(u, A, rhs, max_inner=10)
+
+    todo = [(f, handle(), torch.zeros_like(rhs)) for f in (cg, mixed)]
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    fill = torch.empty(free - (24 << 20), device="cuda", dtype=torch.uint8)
+    got = [f(A, u) for f, A, u in todo]
+    del fill
+    torch.cuda.empty_cache()
+    A = handle()
+    for (f, B, u), st in zip(todo, got):
+        v = torch.zeros_like(rhs)
+        assert f(A, v) == st
+        assert torch.equal(u, v)
+        B.mesh.close()
+    A.mesh.close()
