@@ -21,6 +21,10 @@
 
 using namespace bief;
 
+// Local index lists of the resident solvers: records, binary32 slots (in
+// pairs), segment slots, segment slots in pairs.
+enum { LI_REC, LI_SLOT, LI_SEG, LI_SEGPAIR, LI_N };
+
 struct bief_handle {
   int dev = 0, npoin = 0, nelem = 0, nelmax = 0, nsm = 0;
   int l2_bytes = 0;  // L2 size of the device (operator-load cache policy)
@@ -89,17 +93,25 @@ struct bief_handle {
   double *d_bpart = nullptr;
   long long bpart_cap = 0;
   // plan of the solvers that keep their search direction in shared memory
-  // (bief_resident.h): 0 not made yet, 1 made, -1 the mesh does not fit
+  // (bief_resident.h): 0 not looked at yet, 1 the nodes are shared out, -1
+  // the mesh has no such form
   int res_state = 0;
   bool res_cl = false;
   ResPart res = {};
-  int res_halo_max = 0, max_deg = 0, max_sgdeg = 0, smem_max = 0;
-  int *d_res_off = nullptr, *d_res_halo = nullptr;
-  unsigned long long *d_res_box = nullptr;  // tagged partial sums of the grid form
-  unsigned *d_res_loc = nullptr;
-  unsigned short *d_seg_li = nullptr, *d_sg_li = nullptr, *d_sg_li2 = nullptr;
+  int res_nhalo = 0, res_halo_max = -1;  // -1: halo not counted yet
   int res_shift = 0;  // binary32 local indices: 0 byte offsets, 2 element numbers
-  ushort2 *d_rec_li = nullptr;
+  int max_deg = 0, max_sgdeg = 0, smem_max = 0;
+  unsigned long long *d_res_box = nullptr;  // tagged partial sums of the grid form
+  int *d_res_off = nullptr;                 // halo offsets
+  // room for the halo and one list, behind d_rec_idx in the same allocation
+  // (none on large meshes); the list that lies there
+  char *d_res_room = nullptr;
+  size_t res_room = 0;
+  int res_in_room = -1;
+  // local index lists by what they stand for, each made at the first solve
+  // that reads it; the first one's memory begins with the halo
+  void *d_res_mem[LI_N] = {}, *d_res_list[LI_N] = {};
+  unsigned res_short = 0;  // lists that there was no memory for
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   float solve_ms = 0.f, matvec_ms = 0.f;
   int mv_pending = 0;
@@ -381,57 +393,61 @@ int build_seg_coefs(bief_handle *h, const double *xa, cudaStream_t st) {
   return BIEF_OK;
 }
 
-static int res_mixed_vecs(const bief_handle *h);
 // ---------------------------------------------------------------------------
-// Plan of the resident solvers: who owns which node and what each block's
-// halo is, made at the first solve that can use it (and again when the
-// dot-product tree's shape or the segment numbering changes).
+// Plan of the resident solvers: who owns which node, what each block's halo
+// is, and the local index of every neighbour.  Made piece by piece, as a
+// solve asks for it: nothing for a method whose kernel does not fit the mesh,
+// and one list for one that does.  It stays until the dot-product tree's
+// shape or the segment numbering changes.
+//
+// An allocation costs 320 us from about 1 MB up, which a short solve on a new
+// mesh would feel: so the first list of meshes up to about 450k nodes lies in
+// memory that came with the mesh.  First GRACJG solve on a mesh, five
+// iterations (us), with every list made at once in memory of its own / so /
+// of a later solve: 1,681 nodes 250 / 209 / 89, 152k 1,123 / 306 / 136, 1.0M
+// 2,049 / 1,110 / 343 (k_cg64, which needs no plan: 177, 218 and 454).
 // ---------------------------------------------------------------------------
+constexpr size_t RES_ROOM_MAX = 16 << 20;
+
+// Bytes behind d_rec_idx: tagged sums and halo offsets, then room for the
+// halo (in the cluster form it has two words per node) and one list.
+static size_t res_head(int nsm) {
+  return sizeof(unsigned long long) * 4 * RES_TAG + ((size_t)nsm + 4) / 4 * 4 * sizeof(int);
+}
+static size_t res_room_bytes(int npoin, size_t nrec) {
+  const size_t room = sizeof(ushort2) * (nrec + 32) +
+                      ((size_t)8 * npoin + (size_t)16 * std::min(npoin, 24576) + 15) / 16 * 16;
+  return room <= RES_ROOM_MAX ? room : 0;
+}
+
 void res_drop(bief_handle *h) {
-  void *bufs[] = {h->d_res_off, h->d_res_halo, h->d_res_loc, h->d_res_box, h->d_seg_li, h->d_sg_li, h->d_sg_li2,
-                  h->d_rec_li};
-  for (void *p : bufs)
-    if (p) cudaFree(p);
-  h->d_res_off = h->d_res_halo = nullptr;
-  h->d_res_loc = nullptr;
-  h->d_res_box = nullptr;
-  h->d_seg_li = h->d_sg_li = h->d_sg_li2 = nullptr;
-  h->d_rec_li = nullptr;
+  for (int l = 0; l < LI_N; ++l) {
+    if (h->d_res_mem[l]) cudaFree(h->d_res_mem[l]);
+    h->d_res_mem[l] = h->d_res_list[l] = nullptr;
+  }
+  h->res_in_room = -1;
+  h->res.halo = nullptr;
+  h->res_short = 0;
+  h->res_halo_max = -1;
   h->res_state = 0;
 }
 
 // Tagged partial sums: 2 halves of G two-word values, cleared before each
 // launch (the tags count from 1).
-static size_t res_box_words(int G) { return G <= RES_TAG ? (size_t)4 * G : 0; }
+static size_t res_box_words(const bief_handle *h) {
+  return !h->res_cl && h->res.G <= RES_TAG ? (size_t)4 * h->res.G : 0;
+}
 
 static int res_clear(bief_handle *h, cudaStream_t s) {
-  if (!h->res_cl && h->res.G <= RES_TAG)
-    CK(cudaMemsetAsync(h->d_res_box, 0, sizeof(unsigned long long) * res_box_words(h->res.G), s));
+  const size_t words = res_box_words(h);
+  if (words) CK(cudaMemsetAsync(h->d_res_box, 0, sizeof(unsigned long long) * words, s));
   return BIEF_OK;
 }
 
-// No plan: frees what there is of one, and the other kernels solve from now on.
-static int res_none(bief_handle *h) {
-  res_drop(h);
+// The nodes' shares (host arithmetic only).
+static void res_shape(bief_handle *h) {
   h->res_state = -1;
-  return BIEF_OK;
-}
-
-// Memory for the plan; false when there is none left, which is no error as
-// the kernels that need no plan can solve.
-template <typename T>
-static bool res_alloc(T **p, size_t n) {
-  if (cudaMalloc((void **)p, sizeof(T) * std::max<size_t>(n, 1)) == cudaSuccess) return true;
-  *p = nullptr;
-  cudaGetLastError();
-  return false;
-}
-
-int res_ensure(bief_handle *h, cudaStream_t st) {
-  if (h->res_state) return BIEF_OK;
-  h->res_state = -1;
-  if (h->max_deg > 255 || h->max_nnb > 255 || (h->has_segments && h->max_sgdeg > 255))
-    return BIEF_OK;
+  if (h->max_deg > 255 || h->max_nnb > 255 || (h->has_segments && h->max_sgdeg > 255)) return;
   ResPart Q = {};
   Q.n = h->npoin;
   Q.G = h->G;
@@ -455,15 +471,63 @@ int res_ensure(bief_handle *h, cudaStream_t st) {
   }
   Q.TP = RES_T / Q.S;
   if (Q.G > h->nsm) Q.V = (Q.G + h->nsm - 1) / h->nsm;
-  if (Q.V > 2) return BIEF_OK;
+  if (Q.V > 2) return;
   Q.NP = Q.V > 1 ? (Q.G + Q.V - 1) / Q.V : Q.G * Q.S;
   Q.own = Q.V * Q.R * Q.TP;
-  if (Q.own > 0xffff) return BIEF_OK;
-  if (!res_alloc(&h->d_res_off, (size_t)Q.NP + 1)) return res_none(h);
-  Q.halo_off = h->d_res_off;
+  if (Q.own > 0xffff) return;
+  h->res = Q;
+  h->res_state = 1;
+}
+
+// Shared memory of a method's kernel with `cache` operator slots in it; the
+// halo counts as empty until it is known.
+enum ResFor { RES_CG, RES_STAB, RES_MIXED };
+static size_t res_bytes(const bief_handle *h, ResFor f, int nvec, int cache) {
+  const int cb = f == RES_MIXED ? 4 : (h->sto == 3 ? 8 : 16);
+  const int ib = f == RES_MIXED || h->sto == 3 ? 2 : 4;
+  const int elt = f == RES_MIXED ? 4 : (f == RES_STAB ? 32 : 8);
+  return res_layout(h->res.own, std::max(h->res_halo_max, 0), h->res.G, h->res_cl, elt, nvec, cb,
+                    ib, cache)
+      .total;
+}
+// k_cgstab_res: grid_reduce's own shared memory (under 2 KB)
+static size_t res_limit(const bief_handle *h, ResFor f) {
+  return (size_t)h->smem_max - (f == RES_STAB ? 4096 : 0);
+}
+// Vectors of the own rows in shared memory: GRACJG R and AD (cluster form: X
+// too), mixed r, q, z and the row sums (always in the cluster form); none
+// when those do not fit.
+static int res_vecs(const bief_handle *h, ResFor f) {
+  const int nvec = f == RES_STAB ? 0 : (f == RES_MIXED ? 4 : (h->res_cl ? 3 : 2));
+  return res_bytes(h, f, nvec, 0) <= res_limit(h, f) ? nvec : 0;
+}
+// Binary32 local indices: byte offsets (0) while those fit 16 bits and the
+// vectors stand in shared memory, else element numbers (2).
+static int res_shift_of(const bief_handle *h) {
+  return 4LL * (h->res.own + std::max(h->res_halo_max, 0)) <= 0xffff && res_vecs(h, RES_MIXED) ? 0
+                                                                                              : 2;
+}
+static bool res_fits(const bief_handle *h, ResFor f) {
+  if (h->res_state != 1) return false;
+  if (f == RES_STAB && (h->res_cl || h->res.V != 1)) return false;
+  const int nvec = res_vecs(h, f);
+  if (h->res_cl && (nvec == 0 || (f == RES_MIXED && res_shift_of(h)))) return false;
+  return res_bytes(h, f, nvec, 0) <= res_limit(h, f);
+}
+
+static size_t res_list_bytes(const bief_handle *h, int l) {
+  switch (l) {
+    case LI_REC: return sizeof(ushort2) * ((size_t)h->nrec + 32);
+    case LI_SLOT: return sizeof(short) * (size_t)h->nseg;
+    case LI_SEG: return sizeof(short) * ((size_t)h->nsg_slots + 32);
+    default: return sizeof(short) * (size_t)h->nsg_slots;
+  }
+}
+
+static PlanP res_plan_params(const bief_handle *h) {
   PlanP A = {};
-  A.Q = Q;
   const bool sg = h->has_segments != 0;
+  A.Q = h->res;
   A.nb_meta = sg ? h->d_sg_meta : h->d_meta;
   A.nb_off = sg ? h->d_sg_off : h->d_seg_off;
   A.nb_col = sg ? h->d_sg_col : h->d_seg_col;
@@ -472,59 +536,95 @@ int res_ensure(bief_handle *h, cudaStream_t st) {
   A.seg_col = h->d_seg_col;
   A.rec_off = h->d_rec_off;
   A.rec_idx = h->d_rec_idx;
+  A.sg_meta = h->d_sg_meta;
+  A.sg_off = h->d_sg_off;
+  A.sg_col = h->d_sg_col;
+  return A;
+}
+
+// Halo sizes; res_state -1 when the mesh's local indices need more than 16
+// bits.
+static int res_count(bief_handle *h, cudaStream_t st) {
+  const int NP = h->res.NP;
+  h->res_state = -1;
+  h->res.halo_off = h->d_res_off;
+  PlanP A = res_plan_params(h);
   A.halo_n = h->d_res_off;
   CK(res_launch_plan(false, A, st));
-  std::vector<int> cnt(Q.NP + 1, 0);
-  CK(cudaMemcpyAsync(cnt.data(), h->d_res_off, sizeof(int) * Q.NP, cudaMemcpyDeviceToHost, st));
+  h->launches++;
+  std::vector<int> cnt(NP + 1, 0);
+  CK(cudaMemcpyAsync(cnt.data(), h->d_res_off, sizeof(int) * NP, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   int total = 0, most = 0;
-  for (int p = 0; p <= Q.NP; ++p) {
-    const int c = p < Q.NP ? cnt[p] : 0;
+  for (int q = 0; q <= NP; ++q) {
+    const int c = q < NP ? cnt[q] : 0;
     most = std::max(most, c);
-    cnt[p] = total;
+    cnt[q] = total;
     total += c;
   }
-  if (Q.own + most > 0xffff) return res_none(h);
-  if ((!h->res_cl && !res_alloc(&h->d_res_box, res_box_words(Q.G))) ||
-      !res_alloc(&h->d_res_halo, (size_t)total) || !res_alloc(&h->d_res_loc, (size_t)total) ||
-      !res_alloc(&h->d_seg_li, (size_t)h->nseg) ||
-      !res_alloc(&h->d_rec_li, (size_t)h->nrec + 32) ||
-      (sg && (!res_alloc(&h->d_sg_li, (size_t)h->nsg_slots + 32) ||
-              !res_alloc(&h->d_sg_li2, (size_t)h->nsg_slots))))
-    return res_none(h);
-  CK(cudaMemcpyAsync(h->d_res_off, cnt.data(), sizeof(int) * (Q.NP + 1), cudaMemcpyHostToDevice,
-                     st));
-  CK(cudaMemsetAsync(h->d_seg_li, 0, sizeof(short) * h->nseg, st));
-  CK(cudaMemsetAsync(h->d_rec_li, 0, sizeof(ushort2) * (h->nrec + 32), st));
-  if (sg) {
-    CK(cudaMemsetAsync(h->d_sg_li, 0, sizeof(short) * (h->nsg_slots + 32), st));
-    CK(cudaMemsetAsync(h->d_sg_li2, 0, sizeof(short) * h->nsg_slots, st));
-  }
-  // binary32 windows: local indices as byte offsets while those fit 16 bits
-  // (and the vectors stand in shared memory: the kernel forms that exist)
-  h->res = Q;
-  h->res_halo_max = most;
-  h->res_shift = 4LL * (Q.own + most) <= 0xffff && res_mixed_vecs(h) ? 0 : 2;
-  A.shift = 2 - h->res_shift;
-  A.halo = h->d_res_halo;
-  A.halo_loc = h->d_res_loc;
-  A.seg_li = h->d_seg_li;
-  A.rec_li = h->d_rec_li;
-  if (sg) {
-    A.sg_li = h->d_sg_li;
-    A.sg_li2 = h->d_sg_li2;
-    A.sg_meta = h->d_sg_meta;
-    A.sg_off = h->d_sg_off;
-    A.sg_col = h->d_sg_col;
-  }
-  CK(res_launch_plan(true, A, st));
+  if (h->res.own + most > 0xffff) return BIEF_OK;
+  CK(cudaMemcpyAsync(h->d_res_off, cnt.data(), sizeof(int) * (NP + 1), cudaMemcpyHostToDevice, st));
   CK(cudaStreamSynchronize(st));
-  h->launches += 2;
-  Q.halo = h->d_res_halo;
-  Q.halo_loc = h->d_res_loc;
-  h->res = Q;
+  h->res_nhalo = total;
   h->res_halo_max = most;
+  h->res_shift = res_shift_of(h);
   h->res_state = 1;
+  return BIEF_OK;
+}
+
+// One list, with the halo ahead of it when it is the first.
+static int res_build(bief_handle *h, int l, cudaStream_t st) {
+  const size_t nh = ((size_t)h->res_nhalo + 3) / 4 * 4, bytes = res_list_bytes(h, l);
+  const size_t halo = h->res.halo ? 0 : sizeof(int) * nh * (h->res_cl ? 2 : 1);
+  char *mem = h->d_res_room;
+  if (h->res_in_room >= 0 || halo + bytes > h->res_room) {
+    // no memory left is no error, as the kernels that need no plan can solve
+    if (cudaMalloc(&h->d_res_mem[l], halo + bytes) != cudaSuccess) {
+      cudaGetLastError();
+      h->d_res_mem[l] = nullptr;
+      h->res_short |= 1u << l;
+      return BIEF_OK;
+    }
+    mem = (char *)h->d_res_mem[l];
+  } else {
+    h->res_in_room = l;
+  }
+  char *at = mem + halo;
+  PlanP A = res_plan_params(h);
+  if (halo) {
+    A.halo = (int *)mem;
+    if (h->res_cl) A.halo_loc = (unsigned *)A.halo + nh;
+  }
+  A.shift = 2 - h->res_shift;
+  if (l == LI_REC) A.rec_li = (ushort2 *)at;
+  if (l == LI_SLOT) A.seg_li = (unsigned short *)at;
+  if (l == LI_SEG) A.sg_li = (unsigned short *)at;
+  if (l == LI_SEGPAIR) A.sg_li2 = (unsigned short *)at;
+  CK(cudaMemsetAsync(at, 0, bytes, st));
+  CK(res_launch_plan(true, A, st));
+  h->launches++;
+  CK(cudaStreamSynchronize(st));  // the next solve may be on another stream
+  if (halo) {
+    h->res.halo = A.halo;
+    h->res.halo_loc = A.halo_loc;
+  }
+  h->d_res_list[l] = at;
+  return BIEF_OK;
+}
+
+// *ok: the resident kernel of a method can run, its plan in place.
+static int res_ensure(bief_handle *h, ResFor f, cudaStream_t st, bool *ok) {
+  *ok = false;
+  if (!h->res_state) res_shape(h);
+  if (!res_fits(h, f)) return BIEF_OK;
+  const int l = f == RES_MIXED ? (h->sto == 3 ? LI_SEGPAIR : LI_SLOT)
+                               : (h->sto == 3 ? LI_SEG : LI_REC);
+  if (h->res_short >> l & 1) return BIEF_OK;
+  int stt;
+  if (h->res_halo_max < 0 && (stt = res_count(h, st))) return stt;
+  if (!res_fits(h, f)) return BIEF_OK;
+  if (!h->d_res_list[l] && (stt = res_build(h, l, st))) return stt;
+  *ok = h->d_res_list[l] != nullptr;
   return BIEF_OK;
 }
 
@@ -661,8 +761,8 @@ ResP res_params(const bief_handle *h, const CP &C, int td) {
   ResP P = {};
   P.Q = h->res;
   P.S = C.S;
-  P.li = h->d_sg_li;
-  P.rli = h->d_rec_li;
+  P.li = (const unsigned short *)h->d_res_list[LI_SEG];
+  P.rli = (const ushort2 *)h->d_res_list[LI_REC];
   P.td = td;
   P.da = C.da;
   P.dsc = C.dsc;
@@ -677,86 +777,50 @@ ResP res_params(const bief_handle *h, const CP &C, int td) {
   return P;
 }
 
-// GRACJG with the search direction in shared memory; *done = false when the
-// mesh's window does not fit (k_cg64 then).
-int res_cg(bief_handle *h, const CgP &C, int td, cudaStream_t s, bool *done) {
-  *done = false;
-  if (h->res_state != 1) return BIEF_OK;
-  const ResPart &Q = h->res;
-  const int cb = h->sto == 3 ? 8 : 16, ib = h->sto == 3 ? 2 : 4;
-  int nvec = h->res_cl ? 3 : 2;  // R, AD (and X) of the own rows
-  auto layout = [&](int cache) {
-    return res_layout(Q.own, h->res_halo_max, Q.G, h->res_cl, 8, nvec, cb, ib, cache).total;
-  };
-  if (layout(0) > (size_t)h->smem_max) {
-    if (h->res_cl) return BIEF_OK;
-    nvec = 0;
-    if (layout(0) > (size_t)h->smem_max) return BIEF_OK;
-  }
+// GRACJG with the search direction in shared memory (after res_ensure).
+int res_cg(bief_handle *h, const CgP &C, int td, cudaStream_t s) {
+  const int per_slot = h->sto == 3 ? 10 : 20;
   ResP P = res_params(h, C, td);
-  P.cache = res_cache_slots(h, layout(0), cb + ib);
+  P.nvec = res_vecs(h, RES_CG);
+  P.cache = res_cache_slots(h, res_bytes(h, RES_CG, P.nvec, 0), per_slot);
   P.nitmax = C.nitmax;
-  P.nvec = nvec;
   P.eps = C.eps;
-  P.keep = res_keep(h, C.S.cs_rec != 0, cb + ib);
+  P.keep = res_keep(h, C.S.cs_rec != 0, per_slot);
   P.r = C.r;
   P.ad = C.ad;
-  CK(res_launch_cg(h->sto, h->res_cl, P, layout(P.cache), s));
+  CK(res_launch_cg(h->sto, h->res_cl, P, res_bytes(h, RES_CG, P.nvec, P.cache), s));
   h->launches++;
-  *done = true;
   return BIEF_OK;
 }
 
 // CGSTAB likewise, in the grid form with one tree block per physical block
 // and four vectors of the window in shared memory.
-int res_cgstab(bief_handle *h, const StabP &C, int td, bool comp, cudaStream_t s, bool *done) {
-  *done = false;
-  if (h->res_state != 1 || h->res_cl || h->res.V != 1) return BIEF_OK;
-  const ResPart &Q = h->res;
-  const int cb = h->sto == 3 ? 8 : 16, ib = h->sto == 3 ? 2 : 4;
-  auto layout = [&](int cache) {
-    return res_layout(Q.own, h->res_halo_max, Q.G, false, 32, 0, cb, ib, cache).total;
-  };
-  const size_t fixed = 4096;  // grid_reduce's own shared memory (under 2 KB)
-  if (layout(0) + fixed > (size_t)h->smem_max) return BIEF_OK;
+int res_cgstab(bief_handle *h, const StabP &C, int td, bool comp, cudaStream_t s) {
+  const int per_slot = h->sto == 3 ? 10 : 20;
+  const size_t own = (size_t)h->smem_max - res_limit(h, RES_STAB);
   ResP P = res_params(h, C, td);
-  P.cache = res_cache_slots(h, layout(0) + fixed, cb + ib);
-  P.smem_limit = h->smem_max - (int)fixed;
+  P.cache = res_cache_slots(h, res_bytes(h, RES_STAB, 0, 0) + own, per_slot);
+  P.smem_limit = (int)res_limit(h, RES_STAB);
   P.nitmax = C.nitmax;
   P.eps = C.eps;
-  P.keep = res_keep(h, C.S.cs_rec != 0, cb + ib);
+  P.keep = res_keep(h, C.S.cs_rec != 0, per_slot);
   P.r = C.r;
   P.ad = C.v0;
   P.tv = C.t;
   P.p0 = C.p;
-  CK(res_launch_cgstab(h->sto, comp, P, layout(P.cache), s));
+  CK(res_launch_cgstab(h->sto, comp, P, res_bytes(h, RES_STAB, 0, P.cache), s));
   h->launches++;
-  *done = true;
   return BIEF_OK;
 }
 
 // The mixed-precision solve likewise: r, q, z and the row sums of the own
 // rows in shared memory when they fit (always in the cluster form), else in
 // global memory.
-static size_t res_mixed_layout(const bief_handle *h, int nvec, int cache) {
-  return res_layout(h->res.own, h->res_halo_max, h->res.G, h->res_cl, 4, nvec, 4, 2, cache).total;
-}
-static int res_mixed_vecs(const bief_handle *h) {
-  return res_mixed_layout(h, 4, 0) <= (size_t)h->smem_max ? 4 : 0;
-}
-bool res_mixed_fits(const bief_handle *h) {
-  if (h->res_state != 1) return false;
-  const int nvec = res_mixed_vecs(h);
-  if (h->res_cl && (nvec == 0 || h->res_shift)) return false;
-  return res_mixed_layout(h, nvec, 0) <= (size_t)h->smem_max;
-}
-
 int res_mixed(bief_handle *h, const MixP &C, int td, cudaStream_t s) {
-  const int nvec = res_mixed_vecs(h);
   ResP P = res_params(h, C, td);
-  P.li = h->sto == 3 ? h->d_sg_li2 : h->d_seg_li;
-  P.cache = res_cache_slots(h, res_mixed_layout(h, nvec, 0), 6) / 64 * 64;
-  P.nvec = nvec;
+  P.li = (const unsigned short *)h->d_res_list[h->sto == 3 ? LI_SEGPAIR : LI_SLOT];
+  P.nvec = res_vecs(h, RES_MIXED);
+  P.cache = res_cache_slots(h, res_bytes(h, RES_MIXED, P.nvec, 0), 6) / 64 * 64;
   P.max_outer = C.max_outer;
   P.max_inner = C.max_inner;
   P.outer_tol = C.outer_tol;
@@ -764,8 +828,8 @@ int res_mixed(bief_handle *h, const MixP &C, int td, cudaStream_t s) {
   P.z = C.z;
   P.ri = C.ri;
   P.q = C.q;
-  CK(res_launch_mixed(h->sto, h->res_cl, nvec == 4, h->res_shift, P,
-                      res_mixed_layout(h, nvec, P.cache), s));
+  CK(res_launch_mixed(h->sto, h->res_cl, P.nvec == 4, h->res_shift, P,
+                      res_bytes(h, RES_MIXED, P.nvec, P.cache), s));
   h->launches++;
   return BIEF_OK;
 }
@@ -982,6 +1046,8 @@ int bief_mesh_create(int npoin, int nelem, int nelmax, const int *ikle, int devi
     for (auto &ev : h->ev)
       if ((e = cudaEventCreate(&ev)) != cudaSuccess) return fail(cuda_fail(e, "cudaEventCreate", __LINE__));
     size_t n = (size_t)npoin, ne = (size_t)nelem;
+    h->res_room = res_room_bytes(npoin, nrec);
+    const size_t room = res_head(h->nsm) + h->res_room;
     if ((st = dalloc(&h->d_ptr, n + 1)) || (st = dalloc(&h->d_ek, 3 * ne)) ||
         (st = dalloc(&h->d_ik, 3 * ne)) || (st = dalloc(&h->d_dm, n)) ||
         (st = dalloc(&h->d_dms, n)) || (st = dalloc(&h->d_dsc, n)) ||
@@ -992,10 +1058,14 @@ int bief_mesh_create(int npoin, int nelem, int nelmax, const int *ikle, int devi
         (st = dalloc(&h->d_p1, n)) || (st = dalloc(&h->d_q, n)) || (st = dalloc(&h->d_err, 1)) ||
         (st = dalloc(&h->d_ctl, 1)) || (st = dalloc(&h->d_meta, n)) ||
         (st = dalloc(&h->d_rec_off, (size_t)nsl + 1)) || (st = dalloc(&h->d_seg_off, (size_t)nsl + 1)) ||
-        (st = dalloc(&h->d_rec_idx, nrec)) || (st = dalloc(&h->d_rec_slot, nrec)) ||
+        (st = dalloc(&h->d_rec_idx, nrec + room / sizeof(int2))) ||
+        (st = dalloc(&h->d_rec_slot, nrec)) ||
         (st = dalloc(&h->d_rec_c, nrec + 32)) || (st = dalloc(&h->d_seg_col, nseg)) ||
         (st = dalloc(&h->d_seg_c, nseg)))
       return fail(st);
+    h->d_res_box = (unsigned long long *)(h->d_rec_idx + nrec);
+    h->d_res_off = (int *)(h->d_res_box + 4 * RES_TAG);
+    h->d_res_room = (char *)h->d_res_box + res_head(h->nsm);
     if (mvf != MV_NONE) {
       const size_t bek = mvf == MV_LOCAL ? sizeof(unsigned short) : sizeof(int);
       const void *hek = mvf == MV_LOCAL ? (const void *)mv_ek16.data() : (const void *)mv_ek32.data();
@@ -1226,11 +1296,12 @@ int bief_solve_dev(bief_handle *h, double *x, double *b, bief_slvcfg *cfg, int f
     P.part = h->d_part;
     P.ctl = h->d_ctl;
     P.timeout_ns = h->timeout_ns;
-    bool done = false;
-    if ((st = res_ensure(h, s))) return st;  // plan outside the timed launch
+    bool res = false;
+    if ((st = res_ensure(h, RES_STAB, s, &res))) return st;  // plan outside the timed launch
     CK(cudaEventRecord(h->ev[0], s));
-    if ((st = res_cgstab(h, P, td, comp, s, &done))) return st;
-    if (!done && (st = launch_coop(h, cgstab_kernel(td, h->sto, comp, h->wide), &P, s))) return st;
+    if ((st = res ? res_cgstab(h, P, td, comp, s)
+                  : launch_coop(h, cgstab_kernel(td, h->sto, comp, h->wide), &P, s)))
+      return st;
   } else if (cfg->slv == 7) {  // GMRES
     if (!h->d_gpart && (st = dalloc(&h->d_gpart, 4 * (size_t)h->G * (GM_MAXK + 1) + 4)))
       return st;
@@ -1335,12 +1406,13 @@ int bief_solve_dev(bief_handle *h, double *x, double *b, bief_slvcfg *cfg, int f
     P.part = h->d_part;
     P.ctl = h->d_ctl;
     P.timeout_ns = h->timeout_ns;
-    bool done = false;
-    if (!comp && (st = res_ensure(h, s))) return st;  // plan outside the timed launch
-    if (!comp && h->res_state == 1 && (st = res_clear(h, s))) return st;
+    bool res = false;
+    if (!comp && (st = res_ensure(h, RES_CG, s, &res))) return st;  // plan outside the timed launch
+    if (res && (st = res_clear(h, s))) return st;
     CK(cudaEventRecord(h->ev[0], s));
-    if (!comp && (st = res_cg(h, P, td, s, &done))) return st;
-    if (!done && (st = launch_coop(h, cg_kernel(td, h->sto, comp, h->wide), &P, s))) return st;
+    if ((st = res ? res_cg(h, P, td, s)
+                  : launch_coop(h, cg_kernel(td, h->sto, comp, h->wide), &P, s)))
+      return st;
   }
   CK(cudaEventRecord(h->ev[1], s));
   CK(cudaMemcpyAsync(h->h_ctl, h->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
@@ -1419,8 +1491,8 @@ int bief_solve_mixed_dev(bief_handle *h, double *x, const double *b, int precon,
     da = h->d_dms;
     bw = h->d_bs;
   }
-  if ((st = res_ensure(h, s))) return st;
-  const bool pair = res_mixed_fits(h);  // slots in pairs for k_mixed_res
+  bool pair = false;  // k_mixed_res, with its slots in pairs
+  if ((st = res_ensure(h, RES_MIXED, s, &pair))) return st;
   if ((st = seg ? build_seg_coefs(h, xm, s) : build_records(h, xm, s))) return st;
   if ((st = build_slots32(h, td, xm, da, pair, s))) return st;
   h->s32_gen = -1;

@@ -72,8 +72,9 @@ __device__ __forceinline__ int res_node(const ResPart &Q, int p, int kk, int t) 
 // outside the block that its rows name are marked in a bitmap held in shared
 // memory, PLAN_W * 32 nodes at a time; their ranks are the halo positions.
 //   FILL = false: halo_n[p] = number of halo nodes;
-//   FILL = true : halo lists, and per slot the 16-bit local index of its
-//                 neighbour (records: one for each of their two vertices).
+//   FILL = true : the halo list when A.halo is given, and one list of 16-bit
+//                 local indices: rec_li (a record's two vertices), seg_li,
+//                 sg_li or sg_li2 (a slot's neighbour).
 // ---------------------------------------------------------------------------
 template <bool FILL>
 __global__ void __launch_bounds__(1024, 1) k_res_plan(PlanP A) {
@@ -181,7 +182,7 @@ __global__ void __launch_bounds__(1024, 1) k_res_plan(PlanP A) {
     if (t == 0) s_run += s_w[31];
     if (FILL) {
 #pragma unroll 1
-      for (int q = t; q < PLAN_W; q += T) {
+      for (int q = t; A.halo && q < PLAN_W; q += T) {
         unsigned m = bits[q];
         int r = rank[q];
         while (m) {
@@ -190,9 +191,11 @@ __global__ void __launch_bounds__(1024, 1) k_res_plan(PlanP A) {
           const int j = (int)(lo + 32LL * q + bit);
           const int at = A.Q.halo_off[p] + r++;
           A.halo[at] = j;
-          int pp, loc;
-          res_local(Q, j, pp, loc);
-          A.halo_loc[at] = ((unsigned)pp << 16) | (unsigned)(loc & 0xffff);
+          if (A.halo_loc) {
+            int pp, loc;
+            res_local(Q, j, pp, loc);
+            A.halo_loc[at] = ((unsigned)pp << 16) | (unsigned)(loc & 0xffff);
+          }
         }
       }
       auto local_of = [&](int j, int &loc) -> bool {  // true when this pass settles it
@@ -203,32 +206,32 @@ __global__ void __launch_bounds__(1024, 1) k_res_plan(PlanP A) {
         return true;
       };
       each_row([&](int i) {
-        const int me = A.meta[i], deg = me & 0xffff, nn = me >> 16;
-        const int b = A.seg_off[i >> 5] + (i & 31), rb = A.rec_off[i >> 5] + (i & 31);
         int loc;
-        // binary32 slots: pairs of indices, slot m of a lane at word m / 2
+        // pairs of indices: slot m of a lane at word m / 2
         auto pair_at = [&](int b0, int m) {
           return 2 * (((b0 - (i & 31)) >> 1) + 32 * (m >> 1) + (i & 31)) + (m & 1);
         };
+        if (A.rec_li) {
+          const int deg = A.meta[i] & 0xffff, b = A.rec_off[i >> 5] + (i & 31);
+#pragma unroll 1
+          for (int m = 0; m < deg; ++m) {
+            const int2 v = A.rec_idx[b + 32 * m];
+            if (local_of(v.x, loc)) A.rec_li[b + 32 * m].x = (unsigned short)loc;
+            if (local_of(v.y, loc)) A.rec_li[b + 32 * m].y = (unsigned short)loc;
+          }
+          return;
+        }
+        const bool mesh = A.seg_li != nullptr;  // the mesh's neighbours, else the segments'
+        const int nn = (mesh ? A.meta : A.sg_meta)[i] >> 16;
+        const int b = (mesh ? A.seg_off : A.sg_off)[i >> 5] + (i & 31);
+        const int *col = mesh ? A.seg_col : A.sg_col;
+        unsigned short *pairs = mesh ? A.seg_li : A.sg_li2;
 #pragma unroll 1
         for (int m = 0; m < nn; ++m)
-          if (local_of(A.seg_col[b + 32 * m], loc))
-            A.seg_li[pair_at(b, m)] = (unsigned short)(loc << A.shift);
-#pragma unroll 1
-        for (int m = 0; m < deg; ++m) {
-          const int2 v = A.rec_idx[rb + 32 * m];
-          if (local_of(v.x, loc)) A.rec_li[rb + 32 * m].x = (unsigned short)loc;
-          if (local_of(v.y, loc)) A.rec_li[rb + 32 * m].y = (unsigned short)loc;
-        }
-        if (A.sg_li) {
-          const int sd = A.sg_meta[i] & 0xffff, sb = A.sg_off[i >> 5] + (i & 31);
-#pragma unroll 1
-          for (int m = 0; m < sd; ++m)
-            if (local_of(A.sg_col[sb + 32 * m], loc)) {
-              A.sg_li[sb + 32 * m] = (unsigned short)loc;
-              A.sg_li2[pair_at(sb, m)] = (unsigned short)(loc << A.shift);
-            }
-        }
+          if (local_of(col[b + 32 * m], loc)) {
+            if (pairs) pairs[pair_at(b, m)] = (unsigned short)(loc << A.shift);
+            else A.sg_li[b + 32 * m] = (unsigned short)loc;
+          }
       });
     }
     own_done = true;

@@ -35,13 +35,14 @@ struct PlanP {
   const int *meta, *seg_off, *seg_col;   // binary32 slots: distinct neighbours
   const int *rec_off;                    // records: meta's low half entries
   const int2 *rec_idx;
-  const int *sg_meta, *sg_off, *sg_col;  // segment slots, when sg_li
+  const int *sg_meta, *sg_off, *sg_col;  // segment slots
   int *halo_n;
-  int *halo;
-  unsigned *halo_loc;
-  unsigned short *seg_li, *sg_li, *sg_li2;  // pairs, single, pairs
-  int shift;  // pairs: 2 = indices as byte offsets into a binary32 window
+  int *halo;           // null: there already
+  unsigned *halo_loc;  // cluster form only
+  // one of these: pairs, single, pairs, records
+  unsigned short *seg_li, *sg_li, *sg_li2;
   ushort2 *rec_li;
+  int shift;  // pairs: 2 = indices as byte offsets into a binary32 window
 };
 
 struct RedShared {

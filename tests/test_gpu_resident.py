@@ -303,3 +303,74 @@ def test_no_memory_for_the_plan():
         assert torch.equal(u, v)
         B.mesh.close()
     A.mesh.close()
+
+
+def _rows_mesh(nx, ny):
+    k = np.arange(nx * ny).reshape(ny, nx)
+    a, b, c, d = (v.ravel() for v in (k[:-1, :-1], k[:-1, 1:], k[1:, 1:], k[1:, :-1]))
+    ik = np.concatenate([np.stack([a, b, c], 1), np.stack([a, c, d], 1)]).astype(np.int32)
+    n = nx * ny
+    mesh = bief.Mesh(ik, n)
+    return bief.Matrix(mesh, np.full(n, 8.0), np.full((3, ik.shape[0]), -0.5), "Q", "S"), n
+
+
+@pytest.mark.parametrize("nx,ny,slv,bps", [(70, 71, 6, 0), (601, 599, 6, 2), (2001, 2001, 1, 0)])
+def test_no_plan_for_a_method_without_the_form(nx, ny, slv, bps):
+    """CGSTAB on a cluster-sized mesh and with two tree blocks per block, and
+    GRACJG on a mesh whose window cannot fit, solve without a plan: the first
+    call launches what later ones do, and holds no memory for it."""
+    import torch
+    A, n = _rows_mesh(nx, ny)
+    if bps:
+        A.mesh.set_blocks_per_sm(bps)
+    b = torch.rand(n, device="cuda", dtype=torch.float64)
+    u = torch.zeros_like(b)
+    cfg = bief.SlvCfg(slv=slv, nitmax=3, precon=2, krylov=0, eps=1e-13, zero=0.0)
+    if slv == 6:  # its vectors are allocated at the first call
+        bief.solve(u, A, b, bief.SlvCfg(slv=7, nitmax=1, precon=2, krylov=2, eps=1e-13, zero=0.0))
+    torch.cuda.synchronize()
+    free, launches = torch.cuda.mem_get_info()[0], []
+    for _ in range(2):
+        before = A.mesh.kernel_launches()
+        bief.solve(u.zero_(), A, b, cfg)
+        launches.append(A.mesh.kernel_launches() - before)
+    assert launches[0] == launches[1]
+    assert torch.cuda.mem_get_info()[0] == free
+    A.mesh.close()
+
+
+def test_plan_holds_one_list_per_kind_of_solve(oracle_mod):
+    """Lists are made as solves ask for them, in any order of the kinds: the
+    halo counted once (with the first), one launch for each list."""
+    x, y, ik = _grid(171, 161)
+    n = x.size
+    dm, xm, b = _problem(oracle_mod, x, y, ik)
+    g1, g2, es, ori = mg.segments(ik, n)
+    cfg = bief.SlvCfg(slv=1, nitmax=20, precon=2, krylov=0, eps=1e-9, zero=0.0)
+
+    def run(A, kind):
+        u = np.zeros(n)
+        before = A.mesh.kernel_launches()
+        if kind == "cg":
+            bief.solve(u, A, b.copy(), cfg)
+        else:
+            bief.solve_mixed(u, A, b, outer_tol=1e-10, max_inner=20)
+        return u, A.mesh.kernel_launches() - before
+
+    want = {}
+    for order in (("cg", "mixed"), ("mixed", "cg")):
+        mesh = bief.Mesh(ik, n)
+        mesh.set_segments(g1, g2)
+        A = bief.Matrix(mesh, dm, xm, "Q", "S")
+        extra = []
+        for storage in ("ebe", "seg"):
+            if storage == "seg":
+                A.to_segments()
+            for kind in order:
+                u, first = run(A, kind)
+                v, later = run(A, kind)
+                extra.append(first - later)
+                np.testing.assert_array_equal(u, v)
+                np.testing.assert_array_equal(u, want.setdefault((storage, kind), u))
+        assert extra == [2, 1, 1, 1]
+        mesh.close()
