@@ -273,6 +273,12 @@ int bief_selftest_timeout(int device, long long timeout_ns);
  * solve, perhaps from another thread, needs. */
 int bief_selftest_smem(int device, int *bytes);
 
+/* Layout of the binary32 slots (no reference counterpart, no device needed):
+ * for slices of 32 rows of the given widths, the slots in all and whether
+ * the slices are rounded up to even widths.  BIEF_ERR_SIZE when the widths as
+ * they are come to more than 2^31 - 1 slots. */
+int bief_selftest_slots(int nslices, const int *width, int *last, int *pairs);
+
 /* Shape of the device dot-product tree: number of blocks and threads per
  * block of the persistent solver kernel. */
 int bief_launch_info(bief_handle *h, int *nblocks, int *nthreads);

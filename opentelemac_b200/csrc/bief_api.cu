@@ -101,6 +101,7 @@ struct bief_handle {
   int res_nhalo = 0, res_halo_max = -1;  // -1: halo not counted yet
   int res_shift = 0;  // binary32 local indices: 0 byte offsets, 2 element numbers
   int max_deg = 0, max_sgdeg = 0, smem_max = 0;
+  bool seg_pairs = false, sg_pairs = false;  // slots in slices of even widths
   unsigned long long *d_res_box = nullptr;  // tagged partial sums of the grid form
   int *d_res_off = nullptr;                 // halo offsets
   // room for the halo and one list, behind d_rec_idx in the same allocation
@@ -142,6 +143,22 @@ struct DevGuard {
     if (prev >= 0) cudaSetDevice(prev);
   }
 };
+
+// First slots of slices of 32 rows of the given widths; false when the last
+// one does not fit 32 bits.  Widths are rounded up to even, as k_mixed_res
+// reads slots in pairs, where that fits and meshes of that size can have its
+// form (65,535 local indices in each of up to 1,024 blocks): *pairs.
+bool slot_offsets(int nsl, const int *width, int *off, bool *pairs) {
+  for (int even = 32LL * nsl <= 0xffffLL * 1024; even >= 0; --even) {
+    long long o = off[0] = 0;
+    int k = 0;
+    for (; k < nsl && o <= 0x7fffffffLL; off[++k] = (int)o)
+      o += 32LL * (even ? (width[k] + 1) & ~1 : width[k]);
+    *pairs = even != 0;
+    if (o <= 0x7fffffffLL) return true;
+  }
+  return false;
+}
 
 int typdia_code(char c) {
   switch (c) {
@@ -511,6 +528,7 @@ static bool res_fits(const bief_handle *h, ResFor f) {
   if (h->res_state != 1) return false;
   if (f == RES_STAB && (h->res_cl || h->res.V != 1)) return false;
   const int nvec = res_vecs(h, f);
+  if (f == RES_MIXED && !(h->sto == 3 ? h->sg_pairs : h->seg_pairs)) return false;
   if (h->res_cl && (nvec == 0 || (f == RES_MIXED && res_shift_of(h)))) return false;
   return res_bytes(h, f, nvec, 0) <= res_limit(h, f);
 }
@@ -928,18 +946,19 @@ int bief_mesh_create(int npoin, int nelem, int nelmax, const int *ikle, int devi
     if (d > 0xffff || nnb[i] > 0x7fff) return BIEF_ERR_SIZE;
     meta[i] = d | (nnb[i] << 16);
   }
+  std::vector<int> ws(nsl, 0);
   for (int sgi = 0; sgi < nsl; ++sgi) {
-    int wr = 0, ws = 0;
+    int wr = 0;
     for (int i = 32 * sgi; i < std::min(npoin, 32 * sgi + 32); ++i) {
       wr = std::max(wr, ptr[i + 1] - ptr[i]);
-      ws = std::max(ws, nnb[i]);
+      ws[sgi] = std::max(ws[sgi], nnb[i]);
     }
-    ws = (ws + 1) & ~1;  // binary32 slots also stand in pairs (bief_resident.h)
-    const long long r = (long long)rec_off[sgi] + 32LL * wr, q = (long long)seg_off[sgi] + 32LL * ws;
-    if (r > 0x7fffffffLL || q > 0x7fffffffLL) return BIEF_ERR_SIZE;
+    const long long r = (long long)rec_off[sgi] + 32LL * wr;
+    if (r > 0x7fffffffLL) return BIEF_ERR_SIZE;
     rec_off[sgi + 1] = (int)r;
-    seg_off[sgi + 1] = (int)q;
   }
+  bool seg_pairs = false;
+  if (!slot_offsets(nsl, ws.data(), seg_off.data(), &seg_pairs)) return BIEF_ERR_SIZE;
   const size_t nrec = (size_t)rec_off[nsl], nseg = (size_t)seg_off[nsl];
   std::vector<int2> rec_idx(nrec, make_int2(0, 0));
   std::vector<uchar2> rec_slot(nrec, make_uchar2(0, 0));
@@ -1026,6 +1045,7 @@ int bief_mesh_create(int npoin, int nelem, int nelmax, const int *ikle, int devi
   h->nelmax = nelmax;
   h->nrec = (long long)nrec;
   h->nseg = (long long)nseg;
+  h->seg_pairs = seg_pairs;
   h->max_nnb = max_nnb;
   for (int i = 0; i < npoin; ++i) h->max_deg = std::max(h->max_deg, ptr[i + 1] - ptr[i]);
   int st = BIEF_OK;
@@ -1981,6 +2001,16 @@ int bief_selftest_smem(int device, int *bytes) {
   return BIEF_OK;
 }
 
+int bief_selftest_slots(int nslices, const int *width, int *last, int *pairs) {
+  if (nslices < 1 || !width || !last || !pairs) return BIEF_ERR_ARGS;
+  std::vector<int> off((size_t)nslices + 1);
+  bool even = false;
+  if (!slot_offsets(nslices, width, off.data(), &even)) return BIEF_ERR_SIZE;
+  *last = off[nslices];
+  *pairs = even;
+  return BIEF_OK;
+}
+
 int bief_launch_info(bief_handle *h, int *nblocks, int *nthreads) {
   if (!h) return BIEF_ERR_ARGS;
   if (nblocks) *nblocks = h->G;
@@ -2066,14 +2096,10 @@ int bief_set_segments(bief_handle *h, int nseg, int maxseg, const int *gloseg) {
   }
   const int nsl = (n + 31) / 32;
   std::vector<int> off(nsl + 1, 0), meta(n);
-  for (int sl = 0; sl < nsl; ++sl) {
-    int w = 0;
-    for (int i = 32 * sl; i < std::min(n, 32 * sl + 32); ++i) w = std::max(w, deg[i]);
-    w = (w + 1) & ~1;  // as the element storage's binary32 slots
-    const long long o = (long long)off[sl] + 32LL * w;
-    if (o > 0x7fffffffLL) return BIEF_ERR_SIZE;
-    off[sl + 1] = (int)o;
-  }
+  std::vector<int> width(nsl, 0);
+  for (int i = 0; i < n; ++i) width[i >> 5] = std::max(width[i >> 5], deg[i]);
+  bool pairs = false;
+  if (!slot_offsets(nsl, width.data(), off.data(), &pairs)) return BIEF_ERR_SIZE;
   for (int i = 0; i < n; ++i) {
     if (deg[i] > 0x7fff) return BIEF_ERR_SIZE;
     meta[i] = deg[i] | (deg[i] << 16);
@@ -2139,6 +2165,7 @@ int bief_set_segments(bief_handle *h, int nseg, int maxseg, const int *gloseg) {
   }
   CK(cudaStreamSynchronize(h->stream));
   h->sg16 = fit16;
+  h->sg_pairs = pairs;
   h->nsg = nseg;
   h->max_sgdeg = *std::max_element(deg.begin(), deg.end());
   h->nsg_slots = (long long)nslot;

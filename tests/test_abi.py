@@ -131,3 +131,29 @@ def test_argument_checks_before_the_library():
         bief._host_in(np.zeros(3), 4, "b")
     a = bief._host_in([1, 2, 3, 4], 4, "b")
     assert a.dtype == np.float64 and a.flags.c_contiguous
+
+
+def test_slot_layout():
+    """Binary32 slots: slices of even widths where that fits 2^31 - 1 slots
+    and the mesh is not too large for the kernel that reads pairs, the widths
+    as they are otherwise; what fits as it is is never refused."""
+    L = _native.lib()
+
+    def slots(width):
+        width = np.ascontiguousarray(width, dtype=np.int32)
+        last, pairs = ctypes.c_int(), ctypes.c_int()
+        st = L.bief_selftest_slots(width.size, width.ctypes.data_as(ctypes.c_void_p),
+                                   ctypes.byref(last), ctypes.byref(pairs))
+        return (st, last.value, pairs.value) if st == 0 else st
+
+    assert slots([6, 7, 0, 1]) == (0, 32 * (6 + 8 + 0 + 2), 1)
+    big = 7_000_000                                    # 224M nodes
+    assert slots(np.full(big, 9)) == (0, 32 * 9 * big, 0)      # 10 would be over
+    assert slots(np.full(big, 10)) == _native.BIEF_ERR_SIZE
+    n = 0xffff * 1024 // 32
+    assert slots(np.full(n, 3)) == (0, 32 * 4 * n, 1)
+    assert slots(np.full(n + 1, 3)) == (0, 32 * 3 * (n + 1), 0)
+    w = np.full(n, 31)                                 # 2^31 - 32,768 slots when rounded
+    assert slots(w) == (0, 32 * 32 * n, 1)
+    w[:1000] = 33                                      # 64,000 more: too many when rounded
+    assert slots(w) == (0, 32 * (31 * n + 2000), 0)
