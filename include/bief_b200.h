@@ -266,6 +266,11 @@ int bief_diri01_dev(bief_handle *h, int nptfr, const int *nbor,
  * device stays usable), another status otherwise.  The solvers use the same
  * wait with a 2 s limit. */
 int bief_selftest_timeout(int device, long long timeout_ns);
+/* The same for the waits of the solvers that keep their search direction in
+ * shared memory: form 0 cluster barrier, 1 tagged partial sums, 2 arrival
+ * counter.  BIEF_ERR_DEVICE_TIMEOUT when every thread of the block came back
+ * from the wait and the timeout is recorded. */
+int bief_selftest_wait(int device, int form, long long timeout_ns);
 
 /* The limit of dynamic shared memory now set for the GRACJG kernel of meshes
  * of a few thousand nodes (no reference counterpart).  It belongs to the

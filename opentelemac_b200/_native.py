@@ -35,8 +35,8 @@ EXPORTS = [
     "bief_kernel_launches", "bief_strerror", "bief_solve_noalloc",
     "bief_batch_solve_mixed_dev", "bief_set_segments", "bief_set_matrix_seg",
     "bief_set_matrix_seg_dev", "bief_ebe_to_seg", "bief_matrix_storage",
-    "bief_selftest_timeout", "bief_selftest_smem", "bief_selftest_slots", "bief_diri01",
-    "bief_diri01_dev",
+    "bief_selftest_timeout", "bief_selftest_smem", "bief_selftest_slots", "bief_selftest_wait",
+    "bief_diri01", "bief_diri01_dev",
 ]
 
 
@@ -103,6 +103,7 @@ def lib():
             "bief_ebe_to_seg": ([vp, vp], i),
             "bief_matrix_storage": ([vp], i),
             "bief_selftest_timeout": ([i, ctypes.c_longlong], i),
+            "bief_selftest_wait": ([i, i, ctypes.c_longlong], i),
             "bief_selftest_smem": ([i, pi], i),
             "bief_selftest_slots": ([i, vp, pi, pi], i),
             "bief_diri01": ([vp, i, vp, vp, i, vp, vp, vp, vp], i),

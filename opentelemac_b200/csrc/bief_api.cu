@@ -1994,6 +1994,27 @@ int bief_selftest_timeout(int device, long long timeout_ns) {
   return host.status == ST_TIMEOUT ? BIEF_ERR_DEVICE_TIMEOUT : BIEF_ERR_CUDA;
 }
 
+int bief_selftest_wait(int device, int form, long long timeout_ns) {
+  if (form < 0 || form > 2 || timeout_ns < 1000000LL || timeout_ns > 5000000000LL)
+    return BIEF_ERR_ARGS;
+  DevGuard g(device);
+  struct Mem {
+    Ctl ctl;
+    double part[4];
+    alignas(16) unsigned long long box[8];
+  } *mem = nullptr, host;
+  CK(cudaMalloc((void **)&mem, sizeof(Mem)));
+  cudaError_t e = cudaMemset(mem, 0, sizeof(Mem));
+  if (e == cudaSuccess) e = res_wait_test(form, &mem->ctl, mem->part, mem->box, timeout_ns);
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  if (e == cudaSuccess) e = cudaMemcpy(&host, mem, sizeof(Mem), cudaMemcpyDeviceToHost);
+  cudaFree(mem);
+  if (e != cudaSuccess) return cuda_fail(e, "selftest", __LINE__);
+  const bool ok = host.ctl.status == ST_TIMEOUT && host.ctl.nit == RES_T &&
+                  (form != 0 || host.ctl.relres == (double)RES_T);
+  return ok ? BIEF_ERR_DEVICE_TIMEOUT : BIEF_ERR_CUDA;
+}
+
 int bief_selftest_smem(int device, int *bytes) {
   if (!bytes) return BIEF_ERR_ARGS;
   DevGuard g(device);

@@ -1612,6 +1612,35 @@ __global__ void __launch_bounds__(MT, 1) k_mixed_res(const __grid_constant__ Res
 }
 
 // ---------------------------------------------------------------------------
+// Self-test of the bounded waits: one block of 1024 threads in a reduction
+// that never completes, as if a warp (cluster form) or another block had
+// stopped.  Every thread must come back with false, after the time limit and
+// with the timeout recorded; ctl->nit counts them.  The cluster form makes a
+// complete reduction first, ctl->relres is its sum.
+// ---------------------------------------------------------------------------
+template <int COM>
+__global__ void __launch_bounds__(RES_T, 1) k_res_wait_test(const __grid_constant__ ResP P) {
+  __shared__ RedShared red;
+  __shared__ unsigned long long box[2 * 32];
+  Comm<COM> M;
+  comm_init(M, P, 1, reinterpret_cast<unsigned char *>(&red),
+            reinterpret_cast<unsigned char *>(box));
+  __syncthreads();
+  const double one = 1.0;
+  double sum = 0.0;
+  if constexpr (COM == COM_CL) {
+    M.template send<true>(&one);
+    if (!M.template wait<true>(sum)) return;
+    if (threadIdx.x == 0) P.ctl->relres = sum;
+    if (threadIdx.x < RES_T - 32) M.template send<true>(&one);
+    else M.done();
+  } else {
+    M.template send<true>(&one);
+  }
+  if (!M.template wait<true>(sum)) atomicAdd(&P.ctl->nit, 1);
+}
+
+// ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
 namespace {
@@ -1712,6 +1741,21 @@ cudaError_t res_launch_mixed(int sto, bool cl, bool vs, int shift, const ResP &P
                              cudaStream_t st) {
   return sto == 3 ? launch_mixed<3>(cl, vs, shift, P, smem, st)
                   : launch_mixed<1>(cl, vs, shift, P, smem, st);
+}
+
+cudaError_t res_wait_test(int form, Ctl *ctl, double *part, unsigned long long *box,
+                          long long timeout_ns) {
+  ResP P = {};
+  P.Q.S = 1;
+  P.Q.G = P.Q.NP = form == COM_CL ? 1 : 2;
+  P.ctl = ctl;
+  P.part = part;
+  P.box = box;
+  P.timeout_ns = timeout_ns;
+  if (form == COM_CL) k_res_wait_test<COM_CL><<<1, RES_T>>>(P);
+  else if (form == COM_TAG) k_res_wait_test<COM_TAG><<<1, RES_T>>>(P);
+  else k_res_wait_test<COM_CNT><<<1, RES_T>>>(P);
+  return cudaGetLastError();
 }
 
 cudaError_t res_smem_limit(int *bytes) {

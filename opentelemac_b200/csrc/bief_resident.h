@@ -122,6 +122,10 @@ cudaError_t res_launch_mixed(int sto, bool cl, bool vs, int shift, const ResP &P
 // can be resident (one probe for all cluster kernels).
 bool res_cluster_fits(int np, int tp, size_t smem);
 
+// One block in a reduction that never completes: form 0 cluster, 1 tagged
+// sums, 2 counter; part: 4 values, box: 8 words, cleared.
+cudaError_t res_wait_test(int form, Ctl *ctl, double *part, unsigned long long *box,
+                          long long timeout_ns);
 // The limit of dynamic shared memory that the cluster form's GRACJG (blocks
 // of at most 512 threads) has now.
 cudaError_t res_smem_limit(int *bytes);
