@@ -306,6 +306,16 @@ int bief_set_blocks_per_sm(bief_handle *h, int blocks_per_sm);
 #define BIEF_MV_BAND   2  /* element index, 16-bit vertex offsets: 8 B per entry       */
 #define BIEF_MV_ANY    3  /* element index and both other vertices: 12 B per entry     */
 int bief_matvec_format(bief_handle *h, int *format);
+/* Form of the kernel that the last solve on this handle ran (-1: none yet).
+ * The bits of the solve are the same in every form. */
+#define BIEF_FORM_GATHER   0  /* neighbours gathered from global memory               */
+#define BIEF_FORM_CLUSTER  1  /* search direction in shared memory: one cluster       */
+#define BIEF_FORM_TAGGED   2  /* ... a grid, reductions by tagged partial sums        */
+#define BIEF_FORM_COUNTER  3  /* ... a grid, reductions by an arrival counter         */
+#define BIEF_FORM_GLOBAL   4  /* + the other vectors in global memory                 */
+#define BIEF_FORM_ELEMENTS 8  /* + binary32 local indices as element numbers          */
+#define BIEF_FORM_TWO     16  /* + two blocks of the dot-product tree per block       */
+int bief_solve_form(bief_handle *h, int *form);
 /* Kernel time (ms, CUDA events recorded around the launch on the stream
  * the call used) of the last solve kernel and of the last matvec kernel.  For
  * bief_matvec_dev, which returns before its kernel ends, the matvec time is

@@ -36,7 +36,7 @@ EXPORTS = [
     "bief_batch_solve_mixed_dev", "bief_set_segments", "bief_set_matrix_seg",
     "bief_set_matrix_seg_dev", "bief_ebe_to_seg", "bief_matrix_storage",
     "bief_selftest_timeout", "bief_selftest_smem", "bief_selftest_slots", "bief_selftest_wait",
-    "bief_diri01", "bief_diri01_dev",
+    "bief_solve_form", "bief_diri01", "bief_diri01_dev",
 ]
 
 
@@ -89,6 +89,7 @@ def lib():
             "bief_wave_coef_grad_dev": ([vp, vp, vp, vp, vp, vp, vp], i),
             "bief_launch_info": ([vp, pi, pi], i),
             "bief_matvec_format": ([vp, pi], i),
+            "bief_solve_form": ([vp, pi], i),
             "bief_set_blocks_per_sm": ([vp, i], i),
             "bief_last_timing": ([vp, ctypes.POINTER(ctypes.c_float),
                                   ctypes.POINTER(ctypes.c_float)], i),

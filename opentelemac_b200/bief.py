@@ -124,6 +124,21 @@ class Mesh:
         _check(_native.lib().bief_matvec_format(self._h, ctypes.byref(f)), "bief_matvec_format")
         return self.MATVEC_FORMATS[f.value]
 
+    SOLVE_FORMS = ("gather", "cluster", "tagged", "counter")
+
+    def solve_form(self):
+        """Form of the kernel that the last solve on this mesh ran: 'gather',
+        or the search direction in shared memory ('cluster', 'tagged' or
+        'counter' for how its blocks reduce) with '+global' (other vectors in
+        global memory), '+elements' (binary32 local indices as element
+        numbers) and '+two' (two tree blocks per block); None before."""
+        f = ctypes.c_int()
+        _check(_native.lib().bief_solve_form(self._h, ctypes.byref(f)), "bief_solve_form")
+        if f.value < 0:
+            return None
+        return self.SOLVE_FORMS[f.value & 3] + "".join(
+            s for bit, s in ((4, "+global"), (8, "+elements"), (16, "+two")) if f.value & bit)
+
     def last_timing(self):
         s, m = ctypes.c_float(), ctypes.c_float()
         _native.lib().bief_last_timing(self._h, ctypes.byref(s), ctypes.byref(m))

@@ -113,6 +113,7 @@ struct bief_handle {
   // that reads it; the first one's memory begins with the halo
   void *d_res_mem[LI_N] = {}, *d_res_list[LI_N] = {};
   unsigned res_short = 0;  // lists that there was no memory for
+  int solve_form = -1;     // BIEF_FORM_* of the last solve
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   float solve_ms = 0.f, matvec_ms = 0.f;
   int mv_pending = 0;
@@ -795,6 +796,17 @@ ResP res_params(const bief_handle *h, const CP &C, int td) {
   return P;
 }
 
+// BIEF_FORM_* of a method's resident kernel.
+static int res_form(const bief_handle *h, ResFor f) {
+  int form = h->res_cl ? BIEF_FORM_CLUSTER
+                       : (h->res.G <= RES_TAG && f != RES_STAB ? BIEF_FORM_TAGGED
+                                                               : BIEF_FORM_COUNTER);
+  if (f != RES_STAB && res_vecs(h, f) == 0) form |= BIEF_FORM_GLOBAL;
+  if (f == RES_MIXED && h->res_shift) form |= BIEF_FORM_ELEMENTS;
+  if (h->res.V > 1) form |= BIEF_FORM_TWO;
+  return form;
+}
+
 // GRACJG with the search direction in shared memory (after res_ensure).
 int res_cg(bief_handle *h, const CgP &C, int td, cudaStream_t s) {
   const int per_slot = h->sto == 3 ? 10 : 20;
@@ -1295,6 +1307,7 @@ int bief_solve_dev(bief_handle *h, double *x, double *b, bief_slvcfg *cfg, int f
     if ((st = dalloc(&h->d_gmv, (size_t)nextra * h->npoin))) return st;
     h->gm_k = (nextra + 1) / 2;
   }
+  h->solve_form = BIEF_FORM_GATHER;
   if (cfg->slv == 6) {  // CGSTAB
     StabP P;
     P.npoin = h->npoin;
@@ -1318,6 +1331,7 @@ int bief_solve_dev(bief_handle *h, double *x, double *b, bief_slvcfg *cfg, int f
     P.timeout_ns = h->timeout_ns;
     bool res = false;
     if ((st = res_ensure(h, RES_STAB, s, &res))) return st;  // plan outside the timed launch
+    if (res) h->solve_form = res_form(h, RES_STAB);
     CK(cudaEventRecord(h->ev[0], s));
     if ((st = res ? res_cgstab(h, P, td, comp, s)
                   : launch_coop(h, cgstab_kernel(td, h->sto, comp, h->wide), &P, s)))
@@ -1429,6 +1443,7 @@ int bief_solve_dev(bief_handle *h, double *x, double *b, bief_slvcfg *cfg, int f
     bool res = false;
     if (!comp && (st = res_ensure(h, RES_CG, s, &res))) return st;  // plan outside the timed launch
     if (res && (st = res_clear(h, s))) return st;
+    if (res) h->solve_form = res_form(h, RES_CG);
     CK(cudaEventRecord(h->ev[0], s));
     if ((st = res ? res_cg(h, P, td, s)
                   : launch_coop(h, cg_kernel(td, h->sto, comp, h->wide), &P, s)))
@@ -1513,6 +1528,7 @@ int bief_solve_mixed_dev(bief_handle *h, double *x, const double *b, int precon,
   }
   bool pair = false;  // k_mixed_res, with its slots in pairs
   if ((st = res_ensure(h, RES_MIXED, s, &pair))) return st;
+  h->solve_form = pair ? res_form(h, RES_MIXED) : BIEF_FORM_GATHER;
   if ((st = seg ? build_seg_coefs(h, xm, s) : build_records(h, xm, s))) return st;
   if ((st = build_slots32(h, td, xm, da, pair, s))) return st;
   h->s32_gen = -1;
@@ -2057,6 +2073,12 @@ int bief_set_blocks_per_sm(bief_handle *h, int blocks_per_sm) {
     h->G = G;
   }
   h->wide = wide;
+  return BIEF_OK;
+}
+
+int bief_solve_form(bief_handle *h, int *form) {
+  if (!h || !form) return BIEF_ERR_ARGS;
+  *form = h->solve_form;
   return BIEF_OK;
 }
 

@@ -374,3 +374,75 @@ def test_plan_holds_one_list_per_kind_of_solve(oracle_mod):
                 np.testing.assert_array_equal(u, want.setdefault((storage, kind), u))
         assert extra == [2, 1, 1, 1]
         mesh.close()
+
+
+def _shuffled(x, y, ik, seed=7):
+    """Nodes and elements in random order."""
+    rng = np.random.default_rng(seed)
+    new_id = rng.permutation(x.size)
+    xs, ys = np.empty_like(x), np.empty_like(y)
+    xs[new_id], ys[new_id] = x, y
+    return xs, ys, new_id[ik[rng.permutation(ik.shape[0])]].astype(np.int32)
+
+
+# GRACJG's and the mixed solve's form, iterations of each: more than two tree
+# rows per thread in the last block (R = 3: no cluster); vectors in global
+# memory; local indices as element numbers; two tree blocks per block
+@pytest.mark.parametrize("nx,ny,shuffle,bps,storage,cg,mixed,its", [
+    (63, 65, False, 0, "ebe", "tagged", "tagged", 40),
+    (983, 25, False, 0, "seg", "tagged", "tagged", 40),
+    (707, 709, True, 0, "ebe", "counter+global", "counter+elements", 10),
+    (1301, 1307, False, 0, "ebe", "counter+global", "counter+global+elements", 10),
+    (1301, 1307, False, 0, "seg", "counter+global", "counter+global+elements", 10),
+    (601, 599, False, 2, "seg", "counter+two", "counter+two", 10),
+    (1301, 1307, False, 2, "ebe", "counter+global+two", "counter+global+elements+two", 10)])
+def test_large_forms_bitexact(oracle_mod, nx, ny, shuffle, bps, storage, cg, mixed, its):
+    x, y, ik = _grid(nx, ny)
+    if shuffle:
+        x, y, ik = _shuffled(x, y, ik)
+    n = x.size
+    dm, xm, b = _problem(oracle_mod, x, y, ik)
+    mesh, A, seg = _stored(oracle_mod, ik, n, dm, xm, "S", storage, bps)
+    assert mesh.solve_form() is None
+    G, T = mesh.launch_info()
+    x0 = np.random.default_rng(5).uniform(-0.1, 0.1, n)
+    cfg = bief.SlvCfg(slv=1, nitmax=its, precon=2, krylov=0, eps=1e-9, zero=0.0)
+    kw = dict(eps=1e-9, nitmax=its, x0=x0, dot_mode=oracle_mod.DOT_BLOCKED, nblocks=G, nthreads=T)
+    with oracle_mod.threads():
+        r = (oracle_mod.solve_seg(seg[0], seg[1], dm, "Q", seg[2], "S", b, **kw) if seg else
+             oracle_mod.solve(ik, dm, "Q", xm, "S", b, **kw))
+    for _ in range(2):
+        u = x0.copy()
+        assert bief.solve(u, A, b.copy(), cfg) == (r["status"], r["nit"], r["relres"])
+        np.testing.assert_array_equal(u, r["x"])
+        assert mesh.solve_form() == cg
+    kw = dict(precon=2, inner_tol=0.1, outer_tol=1e-10, max_outer=1000, max_inner=its, nblocks=G,
+              nthreads=T)
+    with oracle_mod.threads():
+        r = (oracle_mod.solve_mixed_seg(seg[0], seg[1], dm, "Q", seg[2], b, **kw) if seg else
+             oracle_mod.solve_mixed(ik, dm, "Q", xm, b, **kw))
+    for _ in range(2):
+        u = np.zeros(n)
+        got = bief.solve_mixed(u, A, b, precon=2, inner_tol=0.1, outer_tol=1e-10, max_inner=its)
+        assert got == (r["status"], r["outer"], r["inner"], r["relres"])
+        np.testing.assert_array_equal(u, r["x"])
+        assert mesh.solve_form() == mixed
+    mesh.close()
+
+
+@pytest.mark.parametrize("nx,ny,kind,form", [
+    (40, 41, "cg", "cluster"), (171, 161, "cg", "tagged"), (225, 221, "cg", "counter"),
+    (40, 41, "mixed", "cluster"), (171, 161, "mixed", "tagged"), (225, 221, "mixed", "counter"),
+    (40, 41, "stab", "gather"), (171, 161, "stab", "counter"), (40, 41, "comp", "gather")])
+def test_form_of_the_last_solve(nx, ny, kind, form):
+    """The sizes of the tests above do run the forms that they are for."""
+    A, n = _rows_mesh(nx, ny)
+    u, b = np.zeros(n), np.ones(n)
+    if kind == "mixed":
+        bief.solve_mixed(u, A, b, max_inner=3)
+    else:
+        cfg = bief.SlvCfg(slv=6 if kind == "stab" else 1, nitmax=3, precon=2, krylov=0, eps=1e-9,
+                          zero=0.0)
+        bief.solve(u, A, b, cfg, modass=3 if kind == "comp" else 1)
+    assert A.mesh.solve_form() == form
+    A.mesh.close()
