@@ -126,6 +126,31 @@ def algorithmic_bytes(npoin, nelem, nseg=None):
     )
 
 
+def solver_bytes(P, form, single):
+    """(kernel, bytes of one iteration) of the kernel that ran: binary64
+    GRACJG, or single: the mixed solve's binary32 iteration.
+
+    'gather': algorithmic_bytes' counts.  With the search direction in shared
+    memory, per operator entry its coefficients and 16-bit local indices
+    (binary64: 20 B per record, 10 B per segment slot; binary32: 6 B per
+    neighbour), whether the entry is read from DRAM, from the L2 or from shared
+    memory, and per node the vectors in global memory: R published and X read
+    and written (binary32: r published); with '+global' also the other reads
+    and writes of R, AD (r, q, z and the row sums); none in a cluster.  Halo
+    values are not counted (2 % at 1M nodes in rows)."""
+    by = algorithmic_bytes(P["npoin"], P["nelem"], P["nseg"])
+    name = "k_mixed" if single else "k_cg"
+    if form.startswith("gather"):
+        return ("k_mixed", by["it32"]) if single else ("k_cg64", by["it64"])
+    n, ne = P["npoin"], P["nelem"]
+    edges = n + ne - 1 if P["nseg"] is None else P["nseg"]   # of a mesh without holes
+    if single:
+        ops, node = 12 * edges, 32 if "+global" in form else 4
+    else:
+        ops, node = (60 * ne if P["nseg"] is None else 20 * edges), 56 if "+global" in form else 24
+    return name + "_res", ops + (0 if form.startswith("cluster") else node * n)
+
+
 class ClockSampler:
     """nvidia-smi clock/throttle samples during the timed region."""
 
@@ -487,19 +512,21 @@ def config2_measure(P2, ws, flush_l2, hbm, steps=2, warmup=1):
 
     cfg = bief.SlvCfg(slv=1, nitmax=1000000, precon=2, krylov=0, eps=eps, zero=0.0)
     f64_ms, f64_kern, f64_res = timed(lambda: bief.solve(x, A, b, cfg))
+    f64_form = mesh.solve_form()
     x64 = x.clone()
     x.zero_()
     tight = bief.SlvCfg(slv=1, nitmax=1000000, precon=2, krylov=0, eps=1e-13, zero=0.0)
     _, nit_t, rel_t = bief.solve(x, A, b, tight)
     x13 = x.clone()
     nrm = lambda v: float(torch.linalg.norm(v))
-    f64_bytes = f64_res[1] * by["it64"]
+    f64_kernel, f64_it = solver_bytes(P2, f64_form, False)
+    f64_bytes = f64_res[1] * f64_it
     out = {"workload": "2001x2001-node P1 mesh, log-uniform depth in [0.5, 500] m (3 "
                        "smoothing passes), relres 1e-10",
            "npoin": P2["npoin"], "nelem": P2["nelem"],
            "persistent_grid": _grid_info(mesh, b.device),
            "fp64": {"ms": f64_ms, "kernel_ms": f64_kern, "iterations": f64_res[1],
-                    "relres": f64_res[2], "kernel": "k_cg64",
+                    "relres": f64_res[2], "kernel": f64_kernel, "form": f64_form,
                     "gbs": f64_bytes / (f64_kern * 1e-3) / 1e9,
                     "frac": f64_bytes / (f64_kern * 1e-3) / 1e9 / hbm,
                     "bytes_per_launch": f64_bytes},
@@ -509,11 +536,12 @@ def config2_measure(P2, ws, flush_l2, hbm, steps=2, warmup=1):
         ms, kern, res = timed(lambda: bief.solve_mixed(x, A, b, precon=2, inner_tol=itol,
                                                        outer_tol=eps))
         st, outer, inner, relres = res
-        mb = inner * by["it32"] + (outer + 1) * by["upd"]
+        kernel, it32 = solver_bytes(P2, mesh.solve_form(), True)
+        mb = inner * it32 + (outer + 1) * by["upd"]
         out[key] = {"ms": ms, "kernel_ms": kern, "inner": inner, "refinements": outer,
                     "relres": relres, "speedup_vs_fp64": f64_ms / ms,
                     "vs_fp64": nrm(x - x64) / nrm(x64), "vs_tight_fp64": nrm(x - x13) / nrm(x13),
-                    "kernel": "k_mixed_res", "gbs": mb / (kern * 1e-3) / 1e9,
+                    "kernel": kernel, "form": mesh.solve_form(), "gbs": mb / (kern * 1e-3) / 1e9,
                     "frac": mb / (kern * 1e-3) / 1e9 / hbm, "bytes_per_launch": mb}
     del x, x64, x13
     return out
@@ -683,13 +711,12 @@ def run_fp64_solve(args, ws, rank, local):
     """Binary64 GRACJG alone on the --n x --n mesh (--depth, --storage,
     --eps, --nitmax): --warmup + --steps solves from x = 0, L2 flushed before
     each, the library's events around the solver launch.  One line: ms per
-    solve and the k_cg64 (or segment) kernel's algorithmic GB/s."""
+    solve and the kernel's GB/s (solver_bytes)."""
     import torch
     from opentelemac_b200 import bief
     torch.cuda.set_device(local)
     dev = torch.device("cuda", local)
     P = build_problem(args.n, local, args.depth, args.storage)
-    by = algorithmic_bytes(P["npoin"], P["nelem"], P["nseg"])
     flush = torch.empty(1024 * 1024 * 1024 // 4, dtype=torch.float32, device=dev)
     clean = torch.ones(256 * 1024 * 1024 // 4, dtype=torch.float32, device=dev)
     x = torch.zeros_like(P["b"])
@@ -704,7 +731,9 @@ def run_fp64_solve(args, ws, rank, local):
             ts.append(P["mesh"].last_timing()[0])
     m = max_over_ranks(statistics.median(ts), ws)
     hbm, src = hbm_peak()
-    gbs = nit * by["it64"] / (m * 1e-3) / 1e9
+    form = P["mesh"].solve_form()
+    it64 = solver_bytes(P, form, False)[1]
+    gbs = nit * it64 / (m * 1e-3) / 1e9
     if rank == 0:
         print(json.dumps({
             "metric": "binary64 GRACJG time-to-solution", "value": m, "unit": "ms",
@@ -715,10 +744,11 @@ def run_fp64_solve(args, ws, rank, local):
                                    f"{args.nitmax}) on the {args.n}x{args.n}-node P1 mesh",
                        "depth": args.depth, "storage": args.storage},
             "iterations": nit, "relres": rel, "ms_per_iteration": m / max(nit, 1),
-            "roofline": {"bound": "hbm", "kernel": "k_cg64", "achieved": gbs, "peak": hbm,
-                         "unit": "GB/s", "frac": gbs / hbm,
+            # (the line's name for binary64 GRACJG; "form" says which kernel ran)
+            "roofline": {"bound": "hbm", "kernel": "k_cg64", "form": form, "achieved": gbs,
+                         "peak": hbm, "unit": "GB/s", "frac": gbs / hbm,
                          "peak_source": f"{src} (MEASURED_PEAKS.json hbm_gbs)",
-                         "bytes_per_iteration": by["it64"]}}), flush=True)
+                         "bytes_per_iteration": it64}}), flush=True)
     P["mesh"].close()
 
 
@@ -805,6 +835,7 @@ def main():
     # binary64 GRACJG (reported beside the headline)
     barrier(ws)
     f64_ms, f64_kern, f64_res = timed(run_fp64, max(2, args.steps // 2), args.warmup)
+    f64_form = mesh.solve_form()
     f64_x_err = float(torch.linalg.norm(x - P["xt"]) / torch.linalg.norm(P["xt"]))
     x_f64 = x.clone()
     nit64 = f64_res[1]
@@ -913,6 +944,7 @@ def main():
         mx_ms, mx_kern, mx_res = timed(run_mixed, args.steps, args.warmup)
     launches = (mesh.kernel_launches() - launches0) * args.steps // (args.steps + args.warmup)
     st, outer, inner, relres = mx_res
+    mixed_form = mesh.solve_form()
     mixed_x_err = float(torch.linalg.norm(x - P["xt"]) / torch.linalg.norm(P["xt"]))
     mixed_vs_f64 = float(torch.linalg.norm(x - x_f64) / torch.linalg.norm(x_f64))
     mixed_vs_tight = float(torch.linalg.norm(x - x_tight) / torch.linalg.norm(x_tight))
@@ -1000,14 +1032,15 @@ def main():
             traffic = json.load(fh)
     except Exception:
         pass
-    mixed_bytes = inner * by["it32"] + (outer + 1) * by["upd"]
+    mixed_kernel, it32 = solver_bytes(P, mixed_form, True)
+    f64_kernel, it64 = solver_bytes(P, f64_form, False)
+    mixed_bytes = inner * it32 + (outer + 1) * by["upd"]
     achieved = mixed_bytes / (kern_ms * 1e-3) / 1e9
-    mixed_traffic = traffic.get("k_mixed_res_bytes_per_launch")
+    mixed_traffic = traffic.get(mixed_kernel + "_bytes_per_launch")
     dram_gbs = mixed_traffic / (kern_ms * 1e-3) / 1e9 if mixed_traffic else None
-    # the binary32 operator and vectors of the 1M-node solve (~96 MB) fit in
-    # the 126 MB L2: whether the launch's working set stays in L2
-    l2_resident = by["mv32"] < 126e6
-    f64_bytes = nit64 * by["it64"]
+    # whether the operator and vectors of an inner iteration stay in the L2
+    l2_resident = it32 < 126e6
+    f64_bytes = nit64 * it64
     mv_gbs = by["mv64"] / (mv_t * 1e-3) / 1e9
     mv32_gbs = by["mv32"] / (mv32_t * 1e-3) / 1e9
 
@@ -1048,22 +1081,24 @@ def main():
             "fp64_modass3": {"ms": sum(c64_ms) / len(c64_ms), "iterations": c64_res[1],
                              "vs_fp64": c64_vs_f64,
                              "note": "GRACJG with compensated dot products (MODASS=3)"},
-            "fp64_cg": {"kernel": "k_cg_res", "gbs": f64_bytes / (f64_kern_ms * 1e-3) / 1e9,
+            "fp64_cg": {"kernel": f64_kernel, "form": f64_form,
+                        "gbs": f64_bytes / (f64_kern_ms * 1e-3) / 1e9,
                         "frac": f64_bytes / (f64_kern_ms * 1e-3) / 1e9 / hbm,
-                        "bytes_per_iteration": by["it64"], "bytes_per_launch": f64_bytes,
-                        "traffic": traffic.get("k_cg_res_bytes_per_launch")},
-            "roofline": {"bound": "hbm", "kernel": "k_mixed_res", "achieved": achieved,
+                        "bytes_per_iteration": it64, "bytes_per_launch": f64_bytes,
+                        "traffic": traffic.get(f64_kernel + "_bytes_per_launch")},
+            "roofline": {"bound": "hbm", "kernel": mixed_kernel, "form": mixed_form,
+                         "achieved": achieved,
                          "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                          "peak_source": f"{peak_src} (MEASURED_PEAKS.json hbm_gbs)",
-                         "bytes_per_launch": mixed_bytes,
+                         "bytes_per_iteration": it32, "bytes_per_launch": mixed_bytes,
                          "traffic": mixed_traffic,
                          "dram_gbs": dram_gbs,
                          "dram_frac": dram_gbs / hbm if dram_gbs else None,
                          "working_set": ("L2-resident: the binary32 operator and vectors "
-                                         "(~96 MB) stay in the 126 MB L2, so frac is "
-                                         "algorithmic bytes over time, not DRAM traffic "
-                                         "(dram_frac); limited by L2 latency and the grid "
-                                         "barriers" if l2_resident else
+                                         "stay in the 126 MB L2 and shared memory, so frac "
+                                         "is bytes read over time, not DRAM traffic "
+                                         "(dram_frac); limited by the latency of the L2 and "
+                                         "the grid reductions" if l2_resident else
                                          "above L2: streamed from HBM")},
             "e2e": {"value": ws * 1000.0 / e2e_ms, "unit": UNIT,
                     "h2d_bytes_per_step": 8 * (npoin + int(xm_h.size)) + 16 * npoin,

@@ -77,3 +77,21 @@ def test_fp64_and_capped_batch_contracts():
              "--steps", "1", "--warmup", "1", timeout=1800)
     assert d["max_inner"] == 40 and d["iterations_rank0"]["max"] == 40
     assert d["converged"] < 256
+
+
+def test_solver_bytes_and_traffic_name_the_kernels_that_run():
+    """The headline's forms have a measured traffic of their own kernel, and a
+    count below the gather kernels' (whose bytes the shared-memory forms do
+    not move)."""
+    sys.path.insert(0, ROOT)
+    import bench
+    P = dict(npoin=1001 * 1001, nelem=2 * 1000 * 1000, nseg=None)
+    with open(os.path.join(ROOT, "profiles", "traffic_1001_ebe_smooth.json")) as fh:
+        traffic = json.load(fh)
+    for single in (False, True):
+        name, nbytes = bench.solver_bytes(P, "counter", single)
+        assert traffic[name + "_bytes_per_launch"] > 0
+        old, gather = bench.solver_bytes(P, "gather", single)
+        assert name == {"k_cg64": "k_cg_res", "k_mixed": "k_mixed_res"}[old]
+        assert bench.solver_bytes(P, "cluster", single)[1] < nbytes < gather
+        assert nbytes < bench.solver_bytes(P, "counter+global", single)[1]
