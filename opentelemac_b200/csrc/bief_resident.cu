@@ -245,9 +245,6 @@ __global__ void __launch_bounds__(1024, 1) k_res_plan(PlanP A) {
 // Reductions.  send() starts one, wait() ends it; work that no other block
 // waits for goes between the two.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void fence_cluster() {
-  asm volatile("fence.acq_rel.cluster;" ::: "memory");
-}
 __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 __device__ __forceinline__ unsigned smem_addr(const void *p) {
   return (unsigned)__cvta_generic_to_shared(p);
@@ -860,7 +857,6 @@ __device__ __forceinline__ void comm_init(Comm<COM> &M, const ResP &P, int V, un
   M.p = blockIdx.x;
   M.nbar = 0;
   if (COM == COM_CL)
-#pragma unroll 1
     if (threadIdx.x == 0) {
       // one arrival per warp of the cluster and reduction
       for (int q = 0; q < 2; ++q)

@@ -50,7 +50,6 @@ struct RedShared {
   double ws[2][32];
   double cold[3];   // scalars of the mixed solve
   double us[2][16];  // alternate: a warp may still read the previous reduction's
-  int err;
 };
 
 struct ResP {
