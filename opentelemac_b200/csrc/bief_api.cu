@@ -428,13 +428,16 @@ int build_seg_coefs(bief_handle *h, const double *xa, cudaStream_t st) {
 constexpr size_t RES_ROOM_MAX = 16 << 20;
 
 // Bytes behind d_rec_idx: tagged sums and halo offsets, then room for the
-// halo (in the cluster form it has two words per node) and one list.
+// halo (in the cluster form it has two words per node) and one list.  A list
+// begins on a 256-byte boundary: a warp's 128 bytes of it then lie in one line
+// (behind a halo of any length, 1.0M nodes: binary64 iteration 4.7 % slower).
+static size_t res_align(size_t bytes) { return (bytes + 255) / 256 * 256; }
 static size_t res_head(int nsm) {
-  return sizeof(unsigned long long) * 4 * RES_TAG + ((size_t)nsm + 4) / 4 * 4 * sizeof(int);
+  return res_align(sizeof(unsigned long long) * 4 * RES_TAG + sizeof(int) * ((size_t)nsm + 1));
 }
 static size_t res_room_bytes(int npoin, size_t nrec) {
-  const size_t room = sizeof(ushort2) * (nrec + 32) +
-                      ((size_t)8 * npoin + (size_t)16 * std::min(npoin, 24576) + 15) / 16 * 16;
+  const size_t room = res_align(sizeof(ushort2) * (nrec + 32)) +
+                      res_align((size_t)8 * npoin + (size_t)16 * std::min(npoin, 24576));
   return room <= RES_ROOM_MAX ? room : 0;
 }
 
@@ -593,8 +596,8 @@ static int res_count(bief_handle *h, cudaStream_t st) {
 
 // One list, with the halo ahead of it when it is the first.
 static int res_build(bief_handle *h, int l, cudaStream_t st) {
-  const size_t nh = ((size_t)h->res_nhalo + 3) / 4 * 4, bytes = res_list_bytes(h, l);
-  const size_t halo = h->res.halo ? 0 : sizeof(int) * nh * (h->res_cl ? 2 : 1);
+  const size_t nh = (size_t)h->res_nhalo, bytes = res_list_bytes(h, l);
+  const size_t halo = h->res.halo ? 0 : res_align(sizeof(int) * nh * (h->res_cl ? 2 : 1));
   char *mem = h->d_res_room;
   if (h->res_in_room >= 0 || halo + bytes > h->res_room) {
     // no memory left is no error, as the kernels that need no plan can solve

@@ -67,7 +67,6 @@ struct ResP {
   long long timeout_ns;
   int cache;                  // operator slots (multiple of 32) kept in shared memory
   int halo_max;
-  int smem_limit;             // most dynamic shared memory a launch of the kernel may have
   int nvec;                   // own-row vectors in shared memory
   // k_cg_res
   int nitmax;
@@ -80,6 +79,7 @@ struct ResP {
   int max_outer, max_inner;
   double outer_tol, inner_tol;
   float *z, *ri, *q;
+  int smem_limit;             // (host) most dynamic shared memory a launch may have
 };
 
 // Shared-memory layout, computed alike by host and kernel.
