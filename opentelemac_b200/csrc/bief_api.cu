@@ -480,7 +480,10 @@ static void res_shape(bief_handle *h) {
     Q.R = std::max(Q.R, (int)((hi - lo + RES_T - 1) / RES_T));
   }
   // Up to RES_MAXCL tree blocks (24,576 nodes): one cluster, each tree block's
-  // warps shared out over as many of its blocks as there are.
+  // warps shared out over as many of its blocks as there are.  Blocks end on
+  // multiples of 32, so the last one of 1,187 of these sizes (4,065 to 4,095
+  // and more from 6,081 on) has up to 2,079 rows, three per thread (R = 3):
+  // those take the grid form.
   h->res_cl = false;
   if (Q.G <= RES_MAXCL && Q.R <= 2) {
     int S = 1;

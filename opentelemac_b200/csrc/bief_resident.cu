@@ -18,8 +18,8 @@
 //   CL = false  one physical block per SM holding V virtual blocks (V = 2
 //               when the tree has more blocks than SMs), grid barriers
 //               through global memory;
-//   CL = true   meshes of up to 12 virtual blocks (24,576 nodes): one cluster
-//               of G*S <= 12 blocks, each holding 1/S of a virtual block's warps;
+//   CL = true   meshes of up to 12 virtual blocks (24,576 nodes) with at most
+//               two rows per thread: one cluster of G*S <= 12 blocks, each holding 1/S of a virtual block's warps;
 //               partial sums and halo values through distributed shared
 //               memory.
 #include <type_traits>
@@ -313,7 +313,9 @@ __device__ __forceinline__ T tag_value(unsigned long long x, unsigned long long 
 // counter 2.5 (1 to 75 blocks) to 2.6 (148); tagged, without / with fences,
 // 17 blocks 1.1 / 1.6, 44 blocks 2.5 / 2.5, 148 blocks 5.5 / 5.3, as polls
 // queue at an L2 line and delay the write they wait for.  So tags up to
-// RES_TAG blocks (23k nodes, 10 blocks: 8.7 against 10.2 us per iteration).
+// RES_TAG blocks: binary64 / mixed us per iteration with tags against the
+// counter, 13 blocks 8.95 / 7.19 against 9.53 / 8.17, 20 blocks (41,000 nodes)
+// 8.98 / 7.75 against 9.55 / 8.18, 24 blocks 9.12 / 7.40 against 9.34 / 8.02.
 //
 // PUB: the reduction also publishes what the block wrote before it (R for
 // its neighbours' halos).  Without it tagged words need no fence: what the
@@ -1318,7 +1320,7 @@ __device__ __noinline__ ResidualSums mixed_residual(const ResP &P, float *s_r) {
 // else in global memory.  SH = 0: local indices as byte offsets.
 // Bound: reductions (5.2 of 12.7 us per iteration at 1.0M nodes; k_mixed 16.4)
 // and the latency of the slots that are not in shared memory; at 4.0M nodes
-// HBM, 184 MB per iteration (78 -> 53 us).
+// HBM, about 200 MB per iteration (78 -> 53 us).
 // ---------------------------------------------------------------------------
 template <int STO, int COM, bool VS, int SH, int MT>
 __global__ void __launch_bounds__(MT, 1) k_mixed_res(const __grid_constant__ ResP P) {
